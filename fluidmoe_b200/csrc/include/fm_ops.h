@@ -71,10 +71,17 @@ int fm_cross_entropy(void* logits, const long long* labels, float* loss_out, int
                      float grad_scale, cudaStream_t s);
 
 // Padded-capacity routing plan (see moe_plan_kernel).  Outputs: sorted_indices [E*cap] int64,
-// slot_probs [E*cap] fp32, slot_of_token [T,k] int32, routed_per_expert [E] int32.
+// slot_probs [E*cap] fp32, slot_of_token [T,k] int32, routed_per_expert [E] int32,
+// tokens_per_expert [E] int32 (== cap; may be null).
 int fm_moe_plan(const long long* top_idx, const float* top_probs, int T, int k, int E, int cap,
                 long long* sorted_indices, float* slot_probs, int* slot_of_token,
-                int* routed_per_expert, cudaStream_t s);
+                int* routed_per_expert, int* tokens_per_expert, cudaStream_t s);
+// Dropless plan of one rank (see dropless_place_kernel): counts / group_rows (padded to 64) /
+// group_offs [E] int32, row_token [rows_max] int64 (-1: zero row, -2: unused), row_prob [rows_max] fp32,
+// slot_of_token [T,k] int32 (row of the pair).  rows_max >= T*k + 63*E.
+int fm_dropless_plan_local(const long long* top_idx, const float* top_probs, int T, int k, int E, int rows_max,
+                           int* counts, int* group_rows, int* group_offs, long long* row_token, float* row_prob,
+                           int* slot_of_token, cudaStream_t s);
 
 // Causal GQA flash attention forward on the packed projection buffer
 // qkv [s, b, G, (qpg + 2) * d] (d == 128): out [s, b, G*qpg, d] bf16, lse [b, G*qpg, s] fp32.

@@ -1,5 +1,5 @@
-// Memory-bound kernels of the layer: normalisation, rotary embedding, router top-k softmax,
-// token permute / un-permute, and the fused Adam step.  All activations are bf16 with fp32
+// Memory-bound kernels of the layer: normalisation, rotary embedding, router backward, token
+// permute / un-permute, and the fused Adam step.  All activations are bf16 with fp32
 // arithmetic; every kernel moves 16 bytes per thread per access and touches each element once
 // where the math allows it.
 #include <cuda_bf16.h>
@@ -278,41 +278,8 @@ __global__ void rope_packed_kernel(__nv_bfloat16* __restrict__ t, const float* _
 }
 
 // --------------------------------------------------------------------------------------------
-// Router: top-k over experts then softmax over the k winners (fp32).  One thread per token.
-// Ties go to the lower expert index.
-// --------------------------------------------------------------------------------------------
-__global__ void topk_softmax_kernel(const float* __restrict__ logits, long long* __restrict__ idx_out,
-                                    float* __restrict__ prob_out, int T, int E, int k) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T) return;
-  const float* l = logits + (long long)t * E;
-  float vals[16];
-  int ids[16];
-  for (int j = 0; j < k; ++j) {
-    float best = -INFINITY;
-    int bi = -1;
-    for (int e = 0; e < E; ++e) {
-      const float v = l[e];
-      bool taken = false;
-      for (int q = 0; q < j; ++q) taken |= (ids[q] == e);
-      if (!taken && (v > best || bi < 0)) {
-        best = v;
-        bi = e;
-      }
-    }
-    vals[j] = best;
-    ids[j] = bi;
-  }
-  float m = vals[0], s = 0.f;
-  for (int j = 0; j < k; ++j) s += __expf(vals[j] - m);
-  for (int j = 0; j < k; ++j) {
-    idx_out[(long long)t * k + j] = ids[j];
-    prob_out[(long long)t * k + j] = __expf(vals[j] - m) / s;
-  }
-}
-
-// --------------------------------------------------------------------------------------------
-// Permute: out[s] = x[idx[s]] (one warp per row, 16-byte accesses).
+// Permute: out[s] = x[idx[s]] (one warp per row, 16-byte accesses); idx -1: a row of zeros, -2: the
+// row is left as it is.
 // --------------------------------------------------------------------------------------------
 __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ x,
                                    const long long* __restrict__ idx,
@@ -322,9 +289,14 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ x,
   const int lane = threadIdx.x & 31;
   for (long long s = (long long)blockIdx.x * warps_per_block + (threadIdx.x >> 5); s < rows;
        s += (long long)gridDim.x * warps_per_block) {
-    const uint4* src = reinterpret_cast<const uint4*>(x + idx[s] * H);
+    const long long from = idx[s];
     uint4* dst = reinterpret_cast<uint4*>(out + s * H);
-    for (int i = lane; i < nvec; i += 32) dst[i] = src[i];
+    if (from >= 0) {
+      const uint4* src = reinterpret_cast<const uint4*>(x + from * H);
+      for (int i = lane; i < nvec; i += 32) dst[i] = src[i];
+    } else if (from == -1) {
+      for (int i = lane; i < nvec; i += 32) dst[i] = make_uint4(0, 0, 0, 0);
+    }
   }
 }
 
@@ -561,150 +533,6 @@ __global__ void router_bwd_kernel(const float* __restrict__ dprobs_slots, const 
 }
 
 // --------------------------------------------------------------------------------------------
-// Routing plan for fixed (padded) capacity.  One CTA per expert:
-//   1. count the tokens routed to the expert;
-//   2. if there are more than `cap`, find the cap-th largest probability by radix select on the
-//      float bits (probabilities are positive, so the unsigned order is the numeric order) and
-//      keep ties in ascending token order;
-//   3. walk the tokens in order and assign slots: kept tokens, plus the first (cap - kept)
-//      tokens that are NOT routed to this expert as padding (probability 0), all in ascending
-//      token order.
-// Outputs have static shapes; nothing is read back by the host.
-// --------------------------------------------------------------------------------------------
-constexpr int kPlanThreads = 512;
-
-__device__ __forceinline__ int block_excl_scan(int v, int* total, int* smem /* [32] */) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  __syncthreads();
-  if (lane == 31) smem[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    int w = lane < kPlanThreads / 32 ? smem[lane] : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += y;
-    }
-    smem[lane] = w;  // inclusive warp totals
-  }
-  __syncthreads();
-  const int base = warp == 0 ? 0 : smem[warp - 1];
-  *total = smem[kPlanThreads / 32 - 1];
-  return base + x - v;
-}
-
-__global__ void __launch_bounds__(kPlanThreads)
-moe_plan_kernel(const long long* __restrict__ top_idx, const float* __restrict__ top_probs, int T,
-                int k, int E, int cap, long long* __restrict__ sorted_indices,
-                float* __restrict__ slot_probs, int* __restrict__ slot_of_token,
-                int* __restrict__ routed_per_expert) {
-  __shared__ int hist[256];
-  __shared__ int scan_s[32];
-  __shared__ int sh_count, sh_prefix, sh_quota;
-  const int e = blockIdx.x;
-  const int tid = threadIdx.x;
-
-  auto lookup = [&](int t, int& j_out) -> float {
-    for (int j = 0; j < k; ++j)
-      if ((int)top_idx[(long long)t * k + j] == e) {
-        j_out = j;
-        return top_probs[(long long)t * k + j];
-      }
-    j_out = -1;
-    return 0.f;
-  };
-
-  // ---- 1. count ----
-  if (tid == 0) sh_count = 0;
-  __syncthreads();
-  int local = 0;
-  for (int t = tid; t < T; t += kPlanThreads) {
-    int j;
-    lookup(t, j);
-    local += j >= 0;
-  }
-  atomicAdd(&sh_count, local);
-  __syncthreads();
-  const int count = sh_count;
-  const int kept_total = min(count, cap);
-
-  // ---- 2. threshold by radix select (only when tokens must be dropped) ----
-  uint32_t thr_bits = 0;   // keep prob > thr, plus `quota` tokens with prob == thr
-  int quota = 0;
-  if (count > cap) {
-    uint32_t prefix = 0, mask = 0;
-    int want = cap;  // rank (1-based, from the top) of the threshold element
-    for (int shift = 24; shift >= 0; shift -= 8) {
-      for (int i = tid; i < 256; i += kPlanThreads) hist[i] = 0;
-      __syncthreads();
-      for (int t = tid; t < T; t += kPlanThreads) {
-        int j;
-        const float pr = lookup(t, j);
-        if (j < 0) continue;
-        const uint32_t b = __float_as_uint(pr);
-        if ((b & mask) == prefix) atomicAdd(&hist[(b >> shift) & 255], 1);
-      }
-      __syncthreads();
-      if (tid == 0) {
-        int acc = 0, bin = 255;
-        for (; bin >= 0; --bin) {
-          if (acc + hist[bin] >= want) break;
-          acc += hist[bin];
-        }
-        sh_prefix = bin;
-        sh_quota = want - acc;  // rank of the threshold inside the chosen bin
-      }
-      __syncthreads();
-      prefix |= (uint32_t)sh_prefix << shift;
-      mask |= 255u << shift;
-      want = sh_quota;
-      __syncthreads();
-    }
-    thr_bits = prefix;
-    quota = want;  // number of elements equal to the threshold that are kept
-  }
-
-  // ---- 3. ordered slot assignment ----
-  int ties_seen = 0, sel_seen = 0, nonrouted_seen = 0;
-  const int pad_budget = cap - kept_total;
-  for (int t0 = 0; t0 < T; t0 += kPlanThreads) {
-    const int t = t0 + tid;
-    int j = -1;
-    float pr = 0.f;
-    bool valid = t < T;
-    if (valid) pr = lookup(t, j);
-    const bool routed = valid && j >= 0;
-    const uint32_t b = __float_as_uint(pr);
-    const bool above = routed && (count <= cap || b > thr_bits);
-    const bool tie = routed && count > cap && b == thr_bits;
-    int tot;
-    const int tie_rank = block_excl_scan(tie ? 1 : 0, &tot, scan_s) + ties_seen;
-    ties_seen += tot;
-    const bool kept = above || (tie && tie_rank < quota);
-    const bool nonrouted = valid && !routed;
-    const int nr_rank = block_excl_scan(nonrouted ? 1 : 0, &tot, scan_s) + nonrouted_seen;
-    nonrouted_seen += tot;
-    const bool selected = kept || (nonrouted && nr_rank < pad_budget);
-    const int pos = block_excl_scan(selected ? 1 : 0, &tot, scan_s) + sel_seen;
-    sel_seen += tot;
-    if (selected && pos < cap) {
-      const long long slot = (long long)e * cap + pos;
-      sorted_indices[slot] = t;
-      slot_probs[slot] = kept ? pr : 0.f;
-      if (kept) slot_of_token[(long long)t * k + j] = (int)slot;
-    }
-    if (routed && !kept) slot_of_token[(long long)t * k + j] = -1;
-  }
-  if (tid == 0) routed_per_expert[e] = kept_total;
-}
-
-// --------------------------------------------------------------------------------------------
 // Cross-entropy over bf16 logits, forward and backward in one kernel: one CTA per row makes one
 // pass for the running max / sum (log-sum-exp) and one pass that overwrites the logits with
 // dlogits = (softmax - onehot) * grad_scale.  Rows whose label is negative are ignored (loss 0,
@@ -861,16 +689,6 @@ extern "C" int fm_rope_packed_gated(void* t, const float* freqs, long long rows,
   return check_launch("rope_packed");
 }
 
-extern "C" int fm_topk_softmax(const float* logits, long long* idx, float* probs, int T, int E,
-                               int k, cudaStream_t s) {
-  if (k > 16 || k > E) {
-    fm_set_error("topk_softmax: k must be at most 16 and at most the number of experts");
-    return -1;
-  }
-  fm::topk_softmax_kernel<<<(T + 127) / 128, 128, 0, s>>>(logits, idx, probs, T, E, k);
-  return check_launch("topk_softmax");
-}
-
 extern "C" int fm_gather_rows(const void* x, const long long* idx, void* out, long long rows, int H,
                               cudaStream_t s) {
   if (H % 8 != 0) {
@@ -975,18 +793,6 @@ extern "C" int fm_adam_background(void* p, const float* g, void* m, void* v, lon
   fm::adam_background_kernel<<<num_ctas, 128, 0, s>>>((bf*)p, g, (bf*)m, (bf*)v, n / 4, lr, beta1, beta2, eps,
                                                      weight_decay, rbc1, rbc2, grad_scale);
   return check_launch("adam_background");
-}
-
-extern "C" int fm_moe_plan(const long long* top_idx, const float* top_probs, int T, int k, int E,
-                           int cap, long long* sorted_indices, float* slot_probs, int* slot_of_token,
-                           int* routed_per_expert, cudaStream_t s) {
-  if (k > 16 || cap > T) {
-    fm_set_error("moe_plan: k must be at most 16 and the capacity at most the number of tokens");
-    return -1;
-  }
-  fm::moe_plan_kernel<<<E, fm::kPlanThreads, 0, s>>>(top_idx, top_probs, T, k, E, cap, sorted_indices,
-                                                    slot_probs, slot_of_token, routed_per_expert);
-  return check_launch("moe_plan");
 }
 
 extern "C" int fm_cross_entropy(void* logits, const long long* labels, float* loss_out, int T, int V,

@@ -61,9 +61,15 @@ void bind_ops(py::module_& m) {
     chk(fm_unpermute_reduce(p<const void*>(rows), p<const int*>(slot), p<const void*>(res),
                             p<void*>(out), T, k, H, st(s)), "unpermute_reduce");
   });
-  m.def("moe_plan", [](u ti, u tp, int T, int k, int E, int cap, u si, u sp, u sot, u rpe, u s) {
+  m.def("moe_plan", [](u ti, u tp, int T, int k, int E, int cap, u si, u sp, u sot, u rpe, u tpe, u s) {
     chk(fm_moe_plan(p<const long long*>(ti), p<const float*>(tp), T, k, E, cap, p<long long*>(si),
-                    p<float*>(sp), p<int*>(sot), p<int*>(rpe), st(s)), "moe_plan");
+                    p<float*>(sp), p<int*>(sot), p<int*>(rpe), p<int*>(tpe), st(s)), "moe_plan");
+  });
+  m.def("dropless_plan_local", [](u ti, u tp, int T, int k, int E, int rows_max, u counts, u rows, u offs, u tok,
+                                  u prob, u sot, u s) {
+    chk(fm_dropless_plan_local(p<const long long*>(ti), p<const float*>(tp), T, k, E, rows_max, p<int*>(counts),
+                               p<int*>(rows), p<int*>(offs), p<long long*>(tok), p<float*>(prob), p<int*>(sot),
+                               st(s)), "dropless_plan_local");
   });
   m.def("flash_attn_fwd", [](u qkv, u out, u lse, int s_, int b, int G, int qpg, int d, float scale,
                              unsigned long long timeout_ns, u status, int version, u s) {

@@ -12,6 +12,12 @@ The reference routes with a fixed padded capacity and drops tokens under imbalan
   direction; the fused device-initiated path does not apply here yet);
 * receiver side: rows are placed expert-major with every expert's run padded to a multiple of 128
   rows of zeros, so that the weight-gradient GEMM can contract in whole 64-row blocks.
+
+With one expert-parallel rank on a GPU there is no exchange, and the plan stays on the device
+(``build_local_plan``): the permuted order IS the expert-major order, padded to 64 rows per expert in a
+buffer sized for the worst case, so that the permute gather writes the rows of the grouped GEMMs (its
+zero rows included) and the un-permute reads theirs.  No host read, no zero fills, no copies between
+the two orders.
 """
 from __future__ import annotations
 
@@ -21,6 +27,7 @@ from typing import List, Optional
 import torch
 import torch.distributed as dist
 
+from .. import _native
 from ..ops import gemm, permute
 from ..parallel import comm
 
@@ -40,6 +47,33 @@ class DroplessPlan:
     rows_em: int                     # rows of the expert-major buffer (padded)
     recv_to_em: torch.Tensor         # [sum(output_splits)] int64: expert-major row of every received row
     routed_per_expert: torch.Tensor  # alias of counts (API symmetry with the padded plan)
+
+
+@dataclass
+class LocalDroplessPlan:
+    """Plan of a single expert-parallel rank, on the device: slots are rows of the expert-major buffer."""
+    sorted_indices: torch.Tensor     # [rows_em] int64 token of every row, -1 zero row, -2 unused row
+    permuted_probs: torch.Tensor     # [rows_em] fp32, 0 for padding
+    slot_of_token: torch.Tensor      # [T, k] int32 row of the j-th choice of token t
+    counts: torch.Tensor             # [E] int32 routed pairs per expert
+    group_rows: torch.Tensor         # [E] int32 counts padded to 64 (the padding rows are computed: zeros)
+    group_offs: torch.Tensor         # [E] int32 first row of every expert
+    rows_em: int
+    routed_per_expert: torch.Tensor  # alias of counts
+
+
+def local_plan_applies(x: torch.Tensor, top_idx: torch.Tensor, w1: torch.Tensor, num_experts: int, ep_group) -> bool:
+    """One rank, and every tensor of a kind that the native gather, GEMM and un-permute kernels take."""
+    return (comm.group_size(ep_group) == 1 and _native.use_native(x, w1) and x.dtype == w1.dtype == torch.bfloat16
+            and x.is_contiguous() and x.shape[1] % 8 == 0 and top_idx.dtype == torch.int64
+            and top_idx.shape[0] > 0 and top_idx.shape[1] <= 16 and num_experts <= 1024
+            and top_idx.numel() + 63 * num_experts < 2 ** 31 - 2 ** 14)
+
+
+def build_local_plan(top_idx: torch.Tensor, top_probs: torch.Tensor, num_experts: int) -> LocalDroplessPlan:
+    from ..ops import elementwise
+    tok, prob, slots, counts, rows, offs = elementwise.dropless_plan_local(top_idx, top_probs, num_experts)
+    return LocalDroplessPlan(tok, prob, slots, counts, rows, offs, tok.numel(), counts)
 
 
 def build_plan(top_idx: torch.Tensor, top_probs: torch.Tensor, num_experts: int, ep_group) -> DroplessPlan:
@@ -88,6 +122,8 @@ def build_plan(top_idx: torch.Tensor, top_probs: torch.Tensor, num_experts: int,
 
 def to_experts(plan: DroplessPlan, rows_permuted: torch.Tensor, ep_group) -> torch.Tensor:
     """Permuted-order rows -> expert-major buffer (zero padded)."""
+    if isinstance(plan, LocalDroplessPlan):
+        return rows_permuted
     if comm.group_size(ep_group) > 1:
         recv = comm.all_to_all(rows_permuted, ep_group, plan.input_splits, plan.output_splits)
     else:
@@ -100,6 +136,8 @@ def to_experts(plan: DroplessPlan, rows_permuted: torch.Tensor, ep_group) -> tor
 
 def from_experts(plan: DroplessPlan, rows_em: torch.Tensor, ep_group) -> torch.Tensor:
     """Expert-major rows -> permuted order on the token owners (the transpose of ``to_experts``)."""
+    if isinstance(plan, LocalDroplessPlan):
+        return rows_em
     send = rows_em.index_select(0, plan.recv_to_em)
     if comm.group_size(ep_group) > 1:
         return comm.all_to_all(send, ep_group, plan.output_splits, plan.input_splits)
@@ -110,23 +148,29 @@ def forward(plan: DroplessPlan, x: torch.Tensor, w1: torch.Tensor, w2: torch.Ten
             ep_group, save_pre: bool = True):
     """Returns ``(combined [T*k, H] in permuted order, state for backward)``."""
     from .moe import MoEForwardState
+    zero_fill = not isinstance(plan, LocalDroplessPlan)      # its unused rows are never read
     permuted = permute.permute_rows(x, plan.sorted_indices)
     tokens_em = to_experts(plan, permuted, ep_group)
     probs_em = to_experts(plan, plan.permuted_probs, ep_group)
     act, pre = gemm.grouped_gemm_act(tokens_em, w1, probs_em, activation=activation,
-                                     group_rows=plan.group_rows, group_offs=plan.group_offs, save_pre=save_pre)
-    out_em = gemm.grouped_gemm(act, w2, b_layout="kn", group_rows=plan.group_rows, group_offs=plan.group_offs)
+                                     group_rows=plan.group_rows, group_offs=plan.group_offs, save_pre=save_pre,
+                                     zero_fill=zero_fill)
+    out_em = gemm.grouped_gemm(act, w2, b_layout="kn", group_rows=plan.group_rows, group_offs=plan.group_offs,
+                               zero_fill=zero_fill)
     return from_experts(plan, out_em, ep_group), MoEForwardState(tokens_em, probs_em, pre, act)
 
 
 def backward(plan: DroplessPlan, grad_combined: torch.Tensor, state, w1: torch.Tensor, w2: torch.Tensor,
              activation: str, ep_group):
     """Returns ``(dfc2_em, dpre_em, dprobs in permuted order, dperm [T*k, H])``."""
+    zero_fill = not isinstance(plan, LocalDroplessPlan)
     dfc2 = to_experts(plan, grad_combined, ep_group)
     dpre, dprobs_em = gemm.grouped_gemm_dact(dfc2, w2, state.pre_em, state.probs_em, activation=activation,
-                                             group_rows=plan.group_rows, group_offs=plan.group_offs)
+                                             group_rows=plan.group_rows, group_offs=plan.group_offs,
+                                             zero_fill=zero_fill)
     dprobs = from_experts(plan, dprobs_em, ep_group)
-    dtok = gemm.grouped_gemm(dpre, w1, b_layout="nk", group_rows=plan.group_rows, group_offs=plan.group_offs)
+    dtok = gemm.grouped_gemm(dpre, w1, b_layout="nk", group_rows=plan.group_rows, group_offs=plan.group_offs,
+                             zero_fill=zero_fill)
     return dfc2, dpre, dprobs, from_experts(plan, dtok, ep_group)
 
 

@@ -159,7 +159,10 @@ class TransformerLayerFunction(torch.autograd.Function):
                         combined, st = fused.dropless.forward(fused._buf(ep), ep, rplan, ln2_out, w1, w2, act,
                                                               save_pre, needs_grad)
                     else:
-                        rplan = moe_dropless.build_plan(top_idx, top_probs, L.num_experts, L.ep_group)
+                        if moe_dropless.local_plan_applies(ln2_out, top_idx, w1, L.num_experts, L.ep_group):
+                            rplan = moe_dropless.build_local_plan(top_idx, top_probs, L.num_experts)
+                        else:
+                            rplan = moe_dropless.build_plan(top_idx, top_probs, L.num_experts, L.ep_group)
                         combined, st = moe_dropless.forward(rplan, ln2_out, w1, w2, act, L.ep_group, save_pre)
             else:
                 gather = not (mode_moe == "fused" and ep.ep_size > 1)

@@ -172,10 +172,33 @@ def moe_plan(top_idx, top_probs, num_experts, capacity):
     slot_probs = torch.empty(num_experts * capacity, dtype=torch.float32, device=dev)
     slot_of_token = torch.empty(T, k, dtype=torch.int32, device=dev)
     routed = torch.empty(num_experts, dtype=torch.int32, device=dev)
+    tpe = torch.empty(num_experts, dtype=torch.int32, device=dev)
     _native.lib().moe_plan(top_idx.data_ptr(), top_probs.data_ptr(), T, k, num_experts, capacity,
                            sorted_indices.data_ptr(), slot_probs.data_ptr(), slot_of_token.data_ptr(),
-                           routed.data_ptr(), _s())
-    return sorted_indices, slot_probs, slot_of_token, routed
+                           routed.data_ptr(), tpe.data_ptr(), _s())
+    return sorted_indices, slot_probs, slot_of_token, routed, tpe
+
+
+def dropless_plan_local(top_idx, top_probs, num_experts):
+    """Expert-major rows of every routed pair, each expert padded to a multiple of 64 rows, without a
+    host read: ``(row_token, row_prob, slot_of_token, counts, group_rows, group_offs)``; the buffer is
+    sized for the worst case, ``row_token`` is -1 for padding and -2 behind the last expert."""
+    global LAUNCHES
+    T, k = top_idx.shape
+    dev = top_idx.device
+    top_idx = top_idx.contiguous()
+    top_probs = top_probs.float().contiguous()
+    rows_max = (T * k + 63 * num_experts + 63) // 64 * 64
+    row_token = torch.empty(rows_max, dtype=torch.int64, device=dev)
+    row_prob = torch.empty(rows_max, dtype=torch.float32, device=dev)
+    slot_of_token = torch.empty(T, k, dtype=torch.int32, device=dev)
+    groups = torch.empty(3, num_experts, dtype=torch.int32, device=dev)
+    counts, group_rows, group_offs = groups[0], groups[1], groups[2]
+    LAUNCHES += 1
+    _native.lib().dropless_plan_local(top_idx.data_ptr(), top_probs.data_ptr(), T, k, num_experts, rows_max,
+                                      counts.data_ptr(), group_rows.data_ptr(), group_offs.data_ptr(),
+                                      row_token.data_ptr(), row_prob.data_ptr(), slot_of_token.data_ptr(), _s())
+    return row_token, row_prob, slot_of_token, counts, group_rows, group_offs
 
 
 def cross_entropy_(logits, labels, grad_scale):

@@ -123,12 +123,15 @@ def grouped_gemm(
     alpha: float = 1.0,
     gate: Optional[dict] = None,
     max_ctas: int = 0,
+    zero_fill: bool = True,
 ) -> torch.Tensor:
     """``out[rows_g] = a[rows_g] @ B_g`` for every group g.
 
     a: [rows, K] bf16.  b: [G, K, N] (``b_layout='kn'``) or [G, N, K] (``'nk'``); a 2-D b is one
     group.  Rows of group g are ``[group_offs[g], group_offs[g] + group_rows[g])`` (device int32
-    tensors, no host sync) or ``uniform_rows`` consecutive rows per group.
+    tensors, no host sync) or ``uniform_rows`` consecutive rows per group.  Rows outside every group
+    are zero in a result allocated here, or undefined when the caller never reads them
+    (``zero_fill=False``, native kernel only).
     """
     b3 = b if b.dim() == 3 else b.unsqueeze(0)
     G = b3.shape[0]
@@ -139,8 +142,8 @@ def grouped_gemm(
         uniform_rows = a.shape[0]
     out_dtype = out_dtype or (out.dtype if out is not None else a.dtype)
     if out is None:
-        out = torch.zeros(a.shape[0], N, dtype=out_dtype, device=a.device) if group_rows is not None \
-            else torch.empty(a.shape[0], N, dtype=out_dtype, device=a.device)
+        holes = group_rows is not None and (zero_fill or not _native.use_native(a, b))
+        out = (torch.zeros if holes else torch.empty)(a.shape[0], N, dtype=out_dtype, device=a.device)
     if not _native.use_native(a, b):
         for g, o, r in _groups(a.shape[0], G, group_rows, group_offs, uniform_rows, group_b):
             if r == 0:
@@ -191,11 +194,13 @@ def grouped_gemm_act(
     gate: Optional[dict] = None,
     act_out: Optional[torch.Tensor] = None,
     pre_out: Optional[torch.Tensor] = None,
+    zero_fill: bool = True,
 ):
     """Expert FC1 with the activation and the routing probability fused into the epilogue.
 
     a: [rows, H]; w: [G, H, F] (or [G, H, 2F] for ``activation='swiglu'``, gate half first);
     probs: fp32 [rows] or None.  Returns ``(act * prob [rows, F], pre-activation or None)``.
+    ``zero_fill``: see ``grouped_gemm``.
     """
     G, H, Fw = w.shape
     gated = activation == "swiglu"
@@ -219,8 +224,7 @@ def grouped_gemm_act(
                 y = y * probs[o:o + r].float().unsqueeze(1)
             act[o:o + r] = y.to(a.dtype)
         return act, pre
-    zeros_needed = group_rows is not None
-    alloc = torch.zeros if zeros_needed else torch.empty
+    alloc = torch.zeros if group_rows is not None and zero_fill else torch.empty
     act = act_out if act_out is not None else alloc(rows, F, dtype=a.dtype, device=a.device)
     pre = pre_out if pre_out is not None else (
         alloc(rows, Fw, dtype=a.dtype, device=a.device) if save_pre else None)
@@ -262,13 +266,15 @@ def grouped_gemm_dact(
     gate: Optional[dict] = None,
     dpre_out: Optional[torch.Tensor] = None,
     dprobs_out: Optional[torch.Tensor] = None,
+    zero_fill: bool = True,
 ):
     """Backward of FC2 and of ``act * prob`` in one kernel.
 
     dy: [rows, H] gradient of the FC2 output; w2: [G, F, H]; pre: saved FC1 pre-activation
     ([rows, F] or [rows, 2F]).  Returns ``(dpre, dprobs fp32 [rows])`` where
     ``dActW = dy @ w2^T``, ``dprobs = sum_F(dActW * act(pre))`` and
-    ``dpre = dActW * prob * act'(pre)`` (fluid/moe/backward.py:341-356).
+    ``dpre = dActW * prob * act'(pre)`` (fluid/moe/backward.py:341-356).  ``zero_fill``: see
+    ``grouped_gemm``.
     """
     G, F, H = w2.shape
     gated = activation == "swiglu"
@@ -293,7 +299,7 @@ def grouped_gemm_dact(
         return dpre, dprobs
     bn = _pick_bn(F)
     nt = (F + bn - 1) // bn
-    alloc = torch.zeros if group_rows is not None else torch.empty
+    alloc = torch.zeros if group_rows is not None and zero_fill else torch.empty
     dpre = dpre_out if dpre_out is not None else alloc(pre.shape, dtype=pre.dtype, device=pre.device)
     partial = torch.zeros(rows, nt * 2, dtype=torch.float32, device=dy.device)
     wflat = w2.reshape(G * F, H)

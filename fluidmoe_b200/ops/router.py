@@ -71,8 +71,7 @@ def build_padded_plan(top_idx: torch.Tensor, top_probs: torch.Tensor, num_expert
     assert capacity <= T, "capacity larger than the number of tokens is not supported"
     if _native.use_native(top_idx, top_probs) and k <= 16:
         from . import elementwise
-        si, sp, sot, routed = elementwise.moe_plan(top_idx, top_probs, E, capacity)
-        tpe = torch.full((E,), capacity, dtype=torch.int32, device=dev)
+        si, sp, sot, routed, tpe = elementwise.moe_plan(top_idx, top_probs, E, capacity)
         return RoutingPlan(si, sp, sot, tpe, routed, None, capacity)
     probs = torch.zeros(T, E, dtype=torch.float32, device=dev).scatter(1, top_idx, top_probs.float())
     rmap = torch.zeros(T, E, dtype=torch.bool, device=dev).scatter(1, top_idx, True)
