@@ -29,7 +29,10 @@ namespace fm {
 constexpr int kBM = 128;
 constexpr int kBK = 64;
 constexpr int kStages = 4;                 // BN = 128; the 256-wide single-CTA tile uses 3
-constexpr int kEpiStageFloats = 32 * 36;   // per epilogue warp: 32 rows x 32 columns, padded rows
+// Staging area of an epilogue warp: two boxes of 32 rows x 128 bytes for bulk tensor stores, or one
+// 32 x 32 fp32 block with padded rows.
+constexpr int kEpiBoxBytes = 32 * 128;
+constexpr int kEpiStageFloats = 2 * kEpiBoxBytes / 4;
 constexpr int kEpiWarps = 8;    // two warps per TMEM lane quarter, each takes half the columns
 constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
 constexpr int kKernelIdGemm = 1;
@@ -200,6 +203,11 @@ struct EpiHasPrefetch { static constexpr bool value = false; };
 template <class E>
 struct EpiHasPrefetch<E, decltype((void)E::kPrefetch)> { static constexpr bool value = true; };
 
+// Tensor maps of the epilogue's outputs, a kernel parameter of its own (the copy engine reads them there).
+struct OutMaps {
+  CUtensorMap m[2];
+};
+
 // No gating: every tile is ready when the kernel starts.
 struct GateNone {
   __device__ __forceinline__ bool wait(const Tile&, const GemmArgs&, volatile int*) const {
@@ -280,7 +288,7 @@ template <bool A_MN, bool B_MN, int BN, class Epi, class Gate>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
                   const __grid_constant__ CUtensorMap tma_b, const GemmArgs args, const Epi epi,
-                  const Gate gate) {
+                  const Gate gate, const __grid_constant__ OutMaps maps) {
   extern __shared__ uint8_t smem_raw[];
   constexpr int A_BYTES = kBM * kBK * 2;
   constexpr int B_BYTES = BN * kBK * 2;
@@ -512,7 +520,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       epi.template run<BN>(t, args, taddr, q * 32 + lane, t.nk == 0, chalf,
-                           epi_stage + (warp - 2) * kEpiStageFloats);
+                           epi_stage + (warp - 2) * kEpiStageFloats, maps.m);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[acc]);
@@ -522,6 +530,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
         acc_phase ^= 1;
       }
     }
+    if (lane == 0) bulk_wait_group<0>();   // the boxes this warp handed to the bulk stores are written
   }
 
   if (*abort_flag) {
@@ -556,7 +565,7 @@ template <bool A_MN, bool B_MN, class Epi, class Gate>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
                    const __grid_constant__ CUtensorMap tma_b, const GemmArgs args, const Epi epi,
-                   const Gate gate) {
+                   const Gate gate, const __grid_constant__ OutMaps maps) {
   constexpr int BN = 256;
   extern __shared__ uint8_t smem_raw[];
   constexpr int A_BYTES = kBM * kBK * 2;          // 128 rows of A
@@ -801,7 +810,7 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       epi.template run<BN>(mine, args, taddr, q * 32 + lane, t.nk == 0, chalf,
-                           epi_stage + (warp - 2) * kEpiStageFloats);
+                           epi_stage + (warp - 2) * kEpiStageFloats, maps.m);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {
@@ -818,6 +827,7 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
       if (lane == 0) ti = order.get(j + 1, seen, timeout, args.status, abort_flag);
       ti = __shfl_sync(0xffffffffu, ti, 0);
     }
+    if (lane == 0) bulk_wait_group<0>();   // the boxes this warp handed to the bulk stores are written
   }
 
   if (*abort_flag) {

@@ -256,3 +256,62 @@ def test_cta_pair_claimed_tile_order_with_row_counts_on_the_device(cta_pair):
         o, r = offs[g].item(), rows[g].item()
         if r:
             _close(out[o:o + r], a[o:o + r].float() @ w[g].float().t())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N,K", [(32, 128, 64), (31, 264, 64), (33, 40, 128), (257, 328, 64), (512, 192, 128)])
+@pytest.mark.parametrize("where", ["whole", "columns", "unaligned"])
+@pytest.mark.parametrize("cta_pair", [0, 1])
+def test_store_writes_its_block_and_nothing_else(dtype, M, N, K, where, cta_pair, monkeypatch):
+    """Bulk tensor stores and the stores from registers they fall back to (partial row blocks, bases off
+    16 bytes) at tile edges; a column block of a wider buffer keeps what lies around it."""
+    monkeypatch.setattr(gemm, "CTA_PAIR", cta_pair)
+    torch.manual_seed(M + N)
+    a, w = _rand(M, K), _rand(N, K)
+    lead = {"whole": 0, "columns": 8, "unaligned": 1}[where]
+    buf = torch.full((M + 2, N + 2 * lead), 7.0, dtype=dtype, device="cuda")
+    if where == "unaligned":
+        buf = torch.full(((M + 2) * (N + 8) + 1,), 7.0, dtype=dtype, device="cuda")[1:].view(M + 2, N + 8)
+    out = buf[1:M + 1, lead:lead + N]
+    gemm.grouped_gemm(a, w, b_layout="nk", out=out, alpha=0.5)
+    torch.cuda.synchronize()
+    gemm.check_status()
+    ref = 0.5 * (a.double() @ w.double().t())
+    # fp32 sums of K products, then one rounding: 2^-8 of the value in bf16
+    tol = (2.0 ** -8 if dtype == torch.bfloat16 else 1e-6) * ref.abs() + 1e-5 * K ** 0.5
+    assert ((out.double() - ref).abs() <= tol).all()
+    keep = torch.ones_like(buf, dtype=torch.bool)
+    keep[1:M + 1, lead:lead + N] = False
+    assert (buf[keep] == 7.0).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("cta_pair", [0, 1])
+def test_stores_of_ragged_groups(dtype, cta_pair, monkeypatch):
+    """Groups that end inside a 32-row block next to rows of the following group, and a weight gradient
+    per group with rows past M cut off."""
+    monkeypatch.setattr(gemm, "CTA_PAIR", cta_pair)
+    torch.manual_seed(3)
+    rows, K, N = [33, 0, 64, 1, 31, 300], 64, 328
+    offs = [0, 33, 33, 97, 98, 129]
+    total = 429 + 16
+    a, w = _rand(total, K), _rand(len(rows), K, N)
+    out = torch.full((total, N), 7.0, dtype=dtype, device="cuda")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
+    gemm.grouped_gemm(a, w, group_rows=i32(rows), group_offs=i32(offs), out=out)
+    for g, (o, r) in enumerate(zip(offs, rows)):
+        ref = a[o:o + r].double() @ w[g].double()
+        tol = (2.0 ** -8 if dtype == torch.bfloat16 else 1e-6) * ref.abs() + 1e-5 * K ** 0.5
+        assert ((out[o:o + r].double() - ref).abs() <= tol).all()
+    assert (out[429:] == 7.0).all()
+    M, G = 200, 3
+    x, dy = _rand(G * 128, M), _rand(G * 128, N)
+    buf = torch.full((G * M * N + 8,), 7.0, dtype=dtype, device="cuda")
+    gw = buf[4 if dtype == torch.float32 else 8:][:G * M * N].view(G, M, N)
+    gemm.grouped_gemm_wgrad(x, dy, G, uniform_rows=128, out=gw)
+    torch.cuda.synchronize()
+    gemm.check_status()
+    ref = x.view(G, 128, M).double().transpose(1, 2) @ dy.view(G, 128, N).double()
+    tol = (2.0 ** -8 if dtype == torch.bfloat16 else 1e-6) * ref.abs() + 1e-5 * 128 ** 0.5
+    assert ((gw.double() - ref).abs() <= tol).all()
+    assert int((buf == 7.0).sum()) >= 8 and (buf[:4] == 7.0).all()
