@@ -267,7 +267,8 @@ struct EpiStore {
 
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
-                                      bool zero, int chalf, float* stg, const CUtensorMap* maps) const {
+                                      bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
+                                      volatile int* abort_flag) const {
     const int lane = r & 31;
     const long long row = a.mode == 0 ? (long long)t.row_base + t.m0 + r : (long long)t.m0 + r;
     const long long row0 = row - lane;   // first row of this warp
@@ -392,6 +393,11 @@ __device__ __forceinline__ void get_block_bf16(float* stg, int lane, float* v, i
 // (12 bytes of traffic per element instead of a 4-byte gradient store here plus a 16-byte
 // optimizer pass later).  Only valid when the gradient is complete after this GEMM: a single
 // micro-batch per step and no data-parallel reduction of this parameter.
+// Bound by memory now (12 bytes an element: 1.7 ms for 8 x 4096 x 28672).  With loads and stores from registers
+// the eight epilogue warps spent their time on the way to L2 (requests 56 % busy, a third of the stalls
+// `lg_throttle`) and on a trip of the accumulator through shared memory; through boxes, with one pipeline
+// stage less, 8 experts of 1024 rows take 3.70 -> 2.69 ms for 4096 x 28672 and 1.78 -> 1.32 ms for
+// 14336 x 4096.
 // ----------------------------------------------------------------------------------------
 struct EpiAdam {
   __nv_bfloat16* P;
@@ -449,6 +455,44 @@ struct EpiAdam {
     }
   }
 
+  int boxes;     // parameter and moments (maps 0 to 2) can be moved by bulk tensor copies
+
+  // Whole blocks (32 rows, all of this warp's columns inside the matrix) are updated in shared memory: boxes
+  // of 32 rows x 32 columns of the three arrays are copied in, read and written back one row per lane,
+  // which is the accumulator's own layout, and copied out.  Two sets of boxes alternate: a set is refilled
+  // while the other is updated.  The 64-byte swizzle (chunk c of row r at c ^ (r >> 1 & 3)) keeps the
+  // 16-byte accesses of eight lanes in different banks.
+  static constexpr int kBox = 32 * 64;
+  static constexpr int kWarpBytes = 2 * 3 * kBox;
+  template <int BN>
+  __device__ __forceinline__ bool whole(const Tile& t, const GemmArgs& a, int r, int chalf) const {
+    // four blocks a tile (BN 256): each set is filled twice, so its barrier's phase starts every tile at 0
+    return BN == 256 && boxes && t.rows_valid - (r & ~31) >= 32 && t.n_tile * BN + (chalf + 1) * (BN / 2) <= a.N;
+  }
+  __device__ __forceinline__ void load_set(const CUtensorMap* maps, uint8_t* set, uint64_t* bar, int col, int row,
+                                           int g) const {
+    mbar_expect_tx(bar, 3 * kBox);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) tma_load_3d(set + i * kBox, maps + i, bar, col, row, g);
+  }
+  template <int BN>
+  __device__ __forceinline__ void fetch(const Tile& t, const GemmArgs& a, int r, int chalf, float* stg,
+                                        const CUtensorMap* maps, uint64_t* wbar) const {
+    if (!whole<BN>(t, a, r, chalf)) return;
+    fence_proxy_async_smem();         // what this warp stored in its area by other means is done
+    __syncwarp();
+    if ((r & 31) == 0) {
+      bulk_wait_group_read<0>();      // the last tile's boxes have left
+      const int row0 = (a.mode == 0 ? t.row_base : 0) + t.m0 + r;
+      const int col = t.n_tile * BN + chalf * (BN / 2);
+      uint8_t* sets = reinterpret_cast<uint8_t*>(stg);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        load_set(maps, sets + i * 3 * kBox, wbar + i, col + 32 * i, row0, a.mode == 0 ? 0 : t.g);
+    }
+    __syncwarp();
+  }
+
   static constexpr bool kPrefetch = true;
   // Called one tile ahead: pull this warp's part of parameter and moments (32 rows x BN/2
   // columns of three bf16 arrays) into L2 while the tensor core still works on the tile.
@@ -472,7 +516,8 @@ struct EpiAdam {
 
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
-                                      bool zero, int chalf, float* stg, const CUtensorMap* maps) const {
+                                      bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
+                                      volatile int* abort_flag) const {
     constexpr int NB = BN / 64;          // 32-column blocks handled by this warp
     const int lane = r & 31;
     const long long row = a.mode == 0 ? (long long)t.row_base + t.m0 + r : (long long)t.m0 + r;
@@ -483,6 +528,50 @@ struct EpiAdam {
     const int sub = lane >> 2, c8 = (lane & 3) * 8;
     const int c_begin = chalf * NB;
     const long long off0 = goff + row0 * ld + (long long)t.n_tile * BN;
+    if (whole<BN>(t, a, r, chalf)) {
+      uint8_t* const sets = reinterpret_cast<uint8_t*>(stg);
+      const int z = a.mode == 0 ? 0 : t.g;
+      const int swz = (lane >> 1) & 3;
+#pragma unroll 1
+      for (int k = 0; k < NB; ++k) {
+        const int col = t.n_tile * BN + (c_begin + k) * 32;
+        uint8_t* const set = sets + (k & 1) * 3 * kBox;
+        float g[32];
+        load_acc(taddr + (c_begin + k) * 32, g, zero);
+        if (lane == 0 && k > 0 && k + 1 < NB) {
+          // the set of the block before has left: refill it for the block after this one
+          bulk_wait_group_read<0>();
+          load_set(maps, sets + ((k + 1) & 1) * 3 * kBox, wbar + ((k + 1) & 1), col + 32, (int)row0, z);
+        }
+        __syncwarp();
+        if (!mbar_wait(wbar + (k & 1), (k >> 1) & 1, a.timeout_ns, abort_flag)) {
+          if (lane == 0) report_status(a.status, kStatusMbarTimeout, kKernelIdGemm2, 500 + k, 0, 0);
+          return;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint4* const at = reinterpret_cast<uint4*>(set + lane * 64 + ((j ^ swz) << 4));
+          uint4 w = at[0], m = at[kBox / 16], v = at[2 * kBox / 16];
+          update8(g + 8 * j, w, m, v);
+          at[0] = w;
+          at[kBox / 16] = m;
+          at[2 * kBox / 16] = v;
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+#pragma unroll
+          for (int i = 0; i < 3; ++i) tma_store_3d(maps + i, set + i * kBox, col, (int)row0, z);
+          bulk_commit_group();
+        }
+      }
+      __syncwarp();
+      return;
+    }
+    if (boxes) {
+      if (lane == 0) bulk_wait_group_read<0>();     // the stage below shares the area with the boxes
+      __syncwarp();
+    }
     // coalesced path: whole 32-column blocks, 16-byte aligned rows (4 lanes x 16 bytes per row)
     const bool vec_ok = (ld & 7) == 0 && aligned16(P + off0) && aligned16(Mo + off0) && aligned16(Vo + off0);
 #pragma unroll 1
@@ -593,7 +682,8 @@ struct EpiAct {
 
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
-                                      bool zero, int chalf, float* stg, const CUtensorMap* maps) const {
+                                      bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
+                                      volatile int* abort_flag) const {
     const int lane = r & 31;
     const long long row = (long long)t.row_base + t.m0 + r;
     const long long row0 = row - lane;
@@ -784,7 +874,8 @@ struct EpiDAct {
 
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
-                                      bool zero, int chalf, float* stg, const CUtensorMap* maps) const {
+                                      bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
+                                      volatile int* abort_flag) const {
     const int lane = r & 31;
     const long long row = (long long)t.row_base + t.m0 + r;
     const long long row0 = row - lane;
@@ -988,7 +1079,8 @@ struct EpiScatter {
 
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
-                                      bool zero, int chalf, float* stg, const CUtensorMap* maps) const {
+                                      bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
+                                      volatile int* abort_flag) const {
     const int lane = r & 31;
     const long long row = (long long)t.row_base + t.m0 + r;
     const bool row_ok = r < t.rows_valid;
@@ -1050,7 +1142,8 @@ struct EpiColScatter {
 
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
-                                      bool zero, int chalf, float* stg, const CUtensorMap* maps) const {
+                                      bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
+                                      volatile int* abort_flag) const {
     const int lane = r & 31;
     const long long row0 = (long long)t.row_base + t.m0 + (r - lane);
     const bool row_ok = r < t.rows_valid;
@@ -1169,9 +1262,9 @@ static bool make_tmap_mn3d(CUtensorMap* m, const void* ptr, long long inner, lon
 }
 
 // Tensor map of an epilogue output [groups][rows][cols] (row stride `ld`, group stride `gs` elements) with
-// boxes of 32 rows x 128 bytes.  False when the addresses or strides do not allow it (16-byte rule).
+// boxes of 32 rows x 128 (or 64) bytes in the swizzle of that width.  False when the addresses or strides do not allow it (16-byte rule).
 static bool make_out_map(CUtensorMap* m, const void* ptr, bool fp32, long long cols, long long rows, long long ld,
-                         long long groups, long long gs) {
+                         long long groups, long long gs, int row_bytes = 128) {
   EncodeTiledFn enc = get_encode();
   const long long es = fp32 ? 4 : 2;
   if (groups <= 1) {
@@ -1184,11 +1277,11 @@ static bool make_out_map(CUtensorMap* m, const void* ptr, bool fp32, long long c
     return false;
   cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)groups};
   cuuint64_t strides[2] = {(cuuint64_t)(ld * es), (cuuint64_t)(gs * es)};
-  cuuint32_t box[3] = {(cuuint32_t)(128 / es), 32, 1};
+  cuuint32_t box[3] = {(cuuint32_t)(row_bytes / es), 32, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   return enc(m, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr),
-             dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-             CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+             dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 static int sm_count() {
@@ -1205,7 +1298,7 @@ template <bool A_MN, bool B_MN, int BN, class Epi, class Gate>
 static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& args,
                       const Epi& epi, const Gate& gate, const OutMaps& maps, int grid, cudaStream_t stream) {
   auto kern = gemm_sm100_kernel<A_MN, B_MN, BN, Epi, Gate>;
-  constexpr int smem = gemm_smem_bytes<BN>();
+  constexpr int smem = gemm_smem_bytes<BN, Epi>();
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -1302,7 +1395,7 @@ template <bool A_MN, bool B_MN, class Epi, class Gate>
 static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& args_in,
                        const Epi& epi, const Gate& gate, const OutMaps& maps, int grid, cudaStream_t stream) {
   auto kern = gemm2_sm100_kernel<A_MN, B_MN, Epi, Gate>;
-  constexpr int smem = gemm2_smem_bytes();
+  constexpr int smem = gemm2_smem_bytes<Epi>();
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -1539,7 +1632,11 @@ extern "C" int fm_gemm_launch(const FmGemmDesc* d, cudaStream_t stream) {
       EpiAdam e{reinterpret_cast<__nv_bfloat16*>(d->adam_p), reinterpret_cast<__nv_bfloat16*>(d->adam_m),
                 reinterpret_cast<__nv_bfloat16*>(d->adam_v), d->ldc, d->c_group_stride,
                 d->alpha == 0.f ? 1.0f : d->alpha, d->adam_lr, d->adam_beta1, d->adam_beta2, d->adam_eps,
-                d->adam_wd, d->adam_rbc1, d->adam_rbc2};
+                d->adam_wd, d->adam_rbc1, d->adam_rbc2, 1};
+      void* const arrays[3] = {d->adam_p, d->adam_m, d->adam_v};
+      for (int i = 0; i < 3; ++i)
+        if (!make_out_map(&maps.m[i], arrays[i], false, d->N, d->M, d->ldc, d->num_groups, d->c_group_stride, 64))
+          e.boxes = 0;
       return dispatch_shape(d, ta, tb, args, e, GateNone{}, maps, grid, stream);
     }
     default:

@@ -205,8 +205,24 @@ struct EpiHasPrefetch<E, decltype((void)E::kPrefetch)> { static constexpr bool v
 
 // Tensor maps of the epilogue's outputs, a kernel parameter of its own (the copy engine reads them there).
 struct OutMaps {
-  CUtensorMap m[2];
+  CUtensorMap m[3];
 };
+
+// An epilogue that updates arrays in place through shared memory declares `static constexpr int
+// kWarpBytes` (staging bytes of a warp) and a member `fetch(tile, args, row, chalf, stg, maps, bars)`, which
+// the epilogue warps call before they wait for the tile's accumulator; `bars` are two barriers of the warp.
+template <class E, class = void>
+struct EpiStaging {
+  static constexpr bool fetches = false;
+  static constexpr int bytes = kEpiStageFloats * 4;
+};
+template <class E>
+struct EpiStaging<E, decltype((void)E::kWarpBytes)> {
+  static constexpr bool fetches = true;
+  static constexpr int bytes = E::kWarpBytes;
+};
+constexpr int kBarBytes = 512;      // pipeline barriers, TMEM slot and abort flag; from byte 256 the warps' own
+constexpr int kWarpBarOffset = 256;
 
 // No gating: every tile is ready when the kernel starts.
 struct GateNone {
@@ -274,14 +290,14 @@ struct GateKSource {
   }
 };
 
-template <int BN>
+template <int BN, class Epi>
 constexpr int gemm_stages() {
-  return BN == 256 ? 3 : 4;
+  return EpiStaging<Epi>::fetches ? (BN == 256 ? 2 : 3) : (BN == 256 ? 3 : 4);
 }
-template <int BN>
+template <int BN, class Epi>
 constexpr int gemm_smem_bytes() {
-  return gemm_stages<BN>() * (kBM * kBK * 2 + BN * kBK * 2) + kEpiWarps * kEpiStageFloats * 4 +
-         1024 /*align*/ + 256 /*barriers*/;
+  return gemm_stages<BN, Epi>() * (kBM * kBK * 2 + BN * kBK * 2) + kEpiWarps * EpiStaging<Epi>::bytes +
+         1024 /*align*/ + kBarBytes;
 }
 
 template <bool A_MN, bool B_MN, int BN, class Epi, class Gate>
@@ -293,14 +309,14 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
   constexpr int A_BYTES = kBM * kBK * 2;
   constexpr int B_BYTES = BN * kBK * 2;
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  constexpr int NSTAGE = gemm_stages<BN>();
+  constexpr int NSTAGE = gemm_stages<BN, Epi>();
   constexpr uint32_t TMEM_COLS = 2 * BN;  // 256 or 512: powers of two
   static_assert(BN == 128 || BN == 256, "BN must be 128 or 256");
 
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* epi_stage = reinterpret_cast<float*>(smem + NSTAGE * STAGE_BYTES);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + NSTAGE * STAGE_BYTES + kEpiWarps * kEpiStageFloats * 4);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + NSTAGE * STAGE_BYTES + kEpiWarps * EpiStaging<Epi>::bytes);
   uint64_t* full = bars;                      // [NSTAGE]
   uint64_t* empty = bars + NSTAGE;           // [NSTAGE]
   uint64_t* tfull = bars + 2 * NSTAGE;       // [2]
@@ -319,6 +335,9 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tfull[i], 1);
       mbar_init(&tempty[i], kEpiWarps);
+    }
+    if constexpr (EpiStaging<Epi>::fetches) {
+      for (int i = 0; i < 2 * kEpiWarps; ++i) mbar_init(&bars[kWarpBarOffset / 8 + i], 1);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -501,6 +520,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
     // ------------------------------- epilogue (8 warps) -------------------------------
     const int q = warp & 3;             // TMEM lane quarter this warp may read
     const int chalf = (warp - 2) >> 2;  // which half of the tile's columns this warp drains
+    float* stg = epi_stage + (warp - 2) * (EpiStaging<Epi>::bytes / 4);
+    uint64_t* wbar = bars + kWarpBarOffset / 8 + 2 * (warp - 2);
     TileWalker<BN> walker(args);
     TileWalker<BN> peek(args);
     Tile t;
@@ -512,6 +533,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
         if (ti == (int)blockIdx.x) epi.template prefetch<BN>(t, args, q * 32 + lane, chalf);
         if (peek.get(ti + gridDim.x, nx)) epi.template prefetch<BN>(nx, args, q * 32 + lane, chalf);
       }
+      if constexpr (EpiStaging<Epi>::fetches) epi.template fetch<BN>(t, args, q * 32 + lane, chalf, stg, maps.m, wbar);
       if (!mbar_wait(&tfull[acc], acc_phase, timeout, abort_flag)) {
         if (lane == 0)
           report_status(args.status, kStatusMbarTimeout, kKernelIdGemm, 400 + acc, 0, 0);
@@ -520,7 +542,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       epi.template run<BN>(t, args, taddr, q * 32 + lane, t.nk == 0, chalf,
-                           epi_stage + (warp - 2) * kEpiStageFloats, maps.m);
+                           stg, maps.m, wbar, abort_flag);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[acc]);
@@ -555,10 +577,13 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
 // completion is broadcast to both CTAs' barriers with tcgen05.commit (multicast of the
 // *arrival*, not of a load).  Each CTA drains its own 128 accumulator rows from its own TMEM.
 // =========================================================================================
-constexpr int kStages2 = 5;
-
+template <class Epi>
+constexpr int gemm2_stages() {
+  return EpiStaging<Epi>::fetches ? 4 : 5;
+}
+template <class Epi>
 constexpr int gemm2_smem_bytes() {
-  return kStages2 * (kBM * kBK * 2 + 128 * kBK * 2) + kEpiWarps * kEpiStageFloats * 4 + 1024 + 256;
+  return gemm2_stages<Epi>() * (kBM * kBK * 2 + 128 * kBK * 2) + kEpiWarps * EpiStaging<Epi>::bytes + 1024 + kBarBytes;
 }
 
 template <bool A_MN, bool B_MN, class Epi, class Gate>
@@ -572,16 +597,17 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
   constexpr int B_BYTES = 128 * kBK * 2;          // this CTA's 128 columns of B
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;  // per CTA
   constexpr uint32_t TMEM_COLS = 2 * BN;
+  constexpr int NSTAGE = gemm2_stages<Epi>();
 
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  float* epi_stage = reinterpret_cast<float*>(smem + kStages2 * STAGE_BYTES);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages2 * STAGE_BYTES + kEpiWarps * kEpiStageFloats * 4);
-  uint64_t* full = bars;                        // [kStages2]  used in the leader CTA
-  uint64_t* empty = bars + kStages2;            // [kStages2]  one per CTA
-  uint64_t* tfull = bars + 2 * kStages2;        // [2]         one per CTA
-  uint64_t* tempty = bars + 2 * kStages2 + 2;   // [2]         used in the leader CTA
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages2 + 4);
+  float* epi_stage = reinterpret_cast<float*>(smem + NSTAGE * STAGE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + NSTAGE * STAGE_BYTES + kEpiWarps * EpiStaging<Epi>::bytes);
+  uint64_t* full = bars;                        // [NSTAGE]  used in the leader CTA
+  uint64_t* empty = bars + NSTAGE;            // [NSTAGE]  one per CTA
+  uint64_t* tfull = bars + 2 * NSTAGE;        // [2]         one per CTA
+  uint64_t* tempty = bars + 2 * NSTAGE + 2;   // [2]         used in the leader CTA
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NSTAGE + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -590,13 +616,16 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
   const bool leader = cta_rank == 0;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages2; ++s) {
+    for (int s = 0; s < NSTAGE; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tfull[i], 1);
       mbar_init(&tempty[i], 2 * kEpiWarps);   // epilogue warps of both CTAs
+    }
+    if constexpr (EpiStaging<Epi>::fetches) {
+      for (int i = 0; i < 2 * kEpiWarps; ++i) mbar_init(&bars[kWarpBarOffset / 8 + i], 1);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -680,7 +709,7 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
           } else {
             tma2_load_3d(sb, &tma_b, &full[stage], 0, t.row_base + k0, n / 64);
           }
-          if (++stage == kStages2) {
+          if (++stage == NSTAGE) {
             stage = 0;
             phase ^= 1;
           }
@@ -753,7 +782,7 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
             umma2_commit_mc(&empty[stage], 3);   // frees the stage in both CTAs
           }
           __syncwarp();
-          if (++stage == kStages2) {
+          if (++stage == NSTAGE) {
             stage = 0;
             phase ^= 1;
           }
@@ -774,6 +803,8 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
     // ------------------------------- epilogue (8 warps per CTA) -------------------------------
     const int q = warp & 3;
     const int chalf = (warp - 2) >> 2;
+    float* stg = epi_stage + (warp - 2) * (EpiStaging<Epi>::bytes / 4);
+    uint64_t* wbar = bars + kWarpBarOffset / 8 + 2 * (warp - 2);
     TileWalker<BN, 2 * kBM> walker(args);
     TileWalker<BN, 2 * kBM> peek(args);
     const TileOrder order(args, pair_id, num_pairs);
@@ -802,6 +833,8 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
           epi.template prefetch<BN>(nx, args, q * 32 + lane, chalf);
         }
       }
+      if constexpr (EpiStaging<Epi>::fetches)
+        epi.template fetch<BN>(mine, args, q * 32 + lane, chalf, stg, maps.m, wbar);
       if (!mbar_wait(&tfull[acc], acc_phase, timeout, abort_flag)) {
         if (lane == 0)
           report_status(args.status, kStatusMbarTimeout, kKernelIdGemm2, 400 + acc, 0, 0);
@@ -810,7 +843,7 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       epi.template run<BN>(mine, args, taddr, q * 32 + lane, t.nk == 0, chalf,
-                           epi_stage + (warp - 2) * kEpiStageFloats, maps.m);
+                           stg, maps.m, wbar, abort_flag);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {

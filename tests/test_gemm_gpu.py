@@ -315,3 +315,32 @@ def test_stores_of_ragged_groups(dtype, cta_pair, monkeypatch):
     tol = (2.0 ** -8 if dtype == torch.bfloat16 else 1e-6) * ref.abs() + 1e-5 * 128 ** 0.5
     assert ((gw.double() - ref).abs() <= tol).all()
     assert int((buf == 7.0).sum()) >= 8 and (buf[:4] == 7.0).all()
+
+
+@pytest.mark.parametrize("G,rows,M,N", [(2, 64, 256, 512), (3, 128, 200, 328), (2, 192, 160, 1024), (1, 64, 8, 264)])
+@pytest.mark.parametrize("cta_pair", [0, 1])
+def test_wgrad_adam_in_boxes_agrees_with_the_path_through_registers(G, rows, M, N, cta_pair, monkeypatch):
+    """Whole blocks move by bulk copies, edges and bases off 16 bytes through registers: results agree to one
+    rounding of bf16 (the unaligned path takes the exact square root and division), and what lies around
+    the arrays stays."""
+    monkeypatch.setattr(gemm, "CTA_PAIR", cta_pair)
+    torch.manual_seed(M)
+    x, dy = _rand(G * rows, M), _rand(G * rows, N)
+    start = [_rand(G, M, N), _rand(G, M, N, scale=0.1), _rand(G, M, N, scale=0.1).abs()]
+    results = []
+    for lead in (8, 1):
+        bufs = [torch.full((G * M * N + 16,), 7.0, dtype=torch.bfloat16, device="cuda") for _ in start]
+        arrays = [b[lead:lead + G * M * N].view(G, M, N) for b in bufs]
+        for a, s in zip(arrays, start):
+            a.copy_(s)
+        for step in (1, 2):
+            gemm.grouped_gemm_wgrad_adam(x, dy, G, *arrays, lr=1e-2, beta1=0.9, beta2=0.99, eps=1e-8,
+                                         weight_decay=0.1, step=step, uniform_rows=rows, grad_scale=0.5)
+        torch.cuda.synchronize()
+        gemm.check_status()
+        for b in bufs:
+            assert (b[:lead] == 7.0).all() and (b[lead + G * M * N:] == 7.0).all()
+        results.append([a.clone() for a in arrays])
+    for s, box, reg in zip(start, *results):
+        assert not torch.equal(s, box)
+        torch.testing.assert_close(box.float(), reg.float(), rtol=2.0 ** -7, atol=1e-6)
