@@ -38,6 +38,27 @@ __device__ __forceinline__ float dact_f(int kind, float x) {
   return kind == FM_ACT_GELU ? dgelu_f(x) : (kind == FM_ACT_SILU ? dsilu_f(x) : 1.0f);
 }
 
+template <int K>
+struct Kind {
+  static constexpr int value = K;
+};
+// Activation and derivative at once: the error function (sigmoid) is evaluated once for both.
+template <int kKind>
+__device__ __forceinline__ void act_dact(float x, float& y, float& dy) {
+  if constexpr (kKind == FM_ACT_GELU) {
+    const float cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
+    y = x * cdf;
+    dy = cdf + x * (0.3989422804014327f * __expf(-0.5f * x * x));
+  } else if constexpr (kKind == FM_ACT_SILU) {
+    const float s = sigmoid_f(x);
+    y = x * s;
+    dy = s * (1.0f + x * (1.0f - s));
+  } else {
+    y = x;
+    dy = 1.0f;
+  }
+}
+
 __device__ __forceinline__ void load_acc(uint32_t taddr, float* v, bool zero) {
   if (zero) {
 #pragma unroll
@@ -219,9 +240,11 @@ struct BoxStore {
     if (lane == 0) bulk_wait_group_read<0>();
     __syncwarp();
   }
-  // The next of the two boxes; the one handed over before the last has been read.
+  // The next of the two boxes.  kPending boxes may still be on their way: 1 when every box is handed over
+  // before the next is opened, 0 when both are open at a time.
+  template <int kPending>
   __device__ __forceinline__ uint8_t* next() {
-    if (lane == 0) bulk_wait_group_read<1>();
+    if (lane == 0) bulk_wait_group_read<kPending>();
     __syncwarp();
     return stg + (n++ & 1) * kEpiBoxBytes;
   }
@@ -293,7 +316,7 @@ struct EpiStore {
 #pragma unroll
               for (int i = 0; i < 32; ++i) v[i] *= alpha;
             }
-            uint8_t* box = bs.next();
+            uint8_t* box = bs.next<1>();
             bs.put_f32(box, v);
             bs.send(maps, box, col, (int)row0, z);
           }
@@ -302,7 +325,7 @@ struct EpiStore {
           for (int c = chalf * kStep; c < (chalf + 1) * kStep; c += 2) {
             const int col = t.n_tile * BN + c * 32;
             if (col >= a.N) break;
-            uint8_t* box = bs.next();
+            uint8_t* box = bs.next<1>();
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               float v[32];
@@ -679,7 +702,9 @@ struct EpiAct {
   long long ld_pre;
   const float* probs;
   int act_kind;
+  int boxes;     // pre-activation (map 0, where it is kept) and activation (map 1) can be written by bulk stores
 
+  // Whole tiles: one row per lane as the accumulator comes, packed into boxes of 64 columns.
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
                                       bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
@@ -690,73 +715,62 @@ struct EpiAct {
     const bool row_ok = r < t.rows_valid;
     const int rows_ok = max(0, min(32, t.rows_valid - (r - lane)));
     const float p = (row_ok && probs) ? probs[row] : 1.0f;
+    const int span = (a.gated ? BN / 2 : BN) / 2;      // output columns of this warp
+    if (boxes && rows_ok == 32 && t.n_tile * 2 * span + (chalf + 1) * span <= a.N) {
+      BoxStore bs(stg, lane);
+      const int c0 = chalf * (span / 32), col0 = t.n_tile * 2 * span + chalf * span;
+#pragma unroll 1
+      for (int c = c0; c < c0 + span / 32; c += 2) {
+        const int col = col0 + (c - c0) * 32;
+        float v[32];
+        if (a.gated) {
+          // three boxes and room for two: the halves are fetched again for the activation
+          if (pre_out != nullptr) {
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              uint8_t* box = bs.next<1>();
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                load_acc(taddr + half * (BN / 2) + (c + h) * 32, v, zero);
+                bs.put_bf16(box, h, v);
+              }
+              bs.send(maps, box, half * a.n_half + col, (int)row0, 0);
+            }
+          }
+          uint8_t* box = bs.next<1>();
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            float u[32];
+            load_acc(taddr + (c + h) * 32, v, zero);
+            load_acc(taddr + BN / 2 + (c + h) * 32, u, zero);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = silu_f(v[i]) * u[i] * p;
+            bs.put_bf16(box, h, v);
+          }
+          bs.send(maps + 1, box, col, (int)row0, 0);
+        } else {
+          uint8_t* box = bs.next<0>();
+          uint8_t* abox = bs.next<0>();
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            load_acc(taddr + (c + h) * 32, v, zero);
+            if (pre_out != nullptr) bs.put_bf16(box, h, v);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = act_f(act_kind, v[i]) * p;
+            bs.put_bf16(abox, h, v);
+          }
+          if (pre_out != nullptr) bs.send(maps, box, col, (int)row0, 0);
+          bs.send(maps + 1, abox, col, (int)row0, 0);
+        }
+      }
+      return;
+    }
+    if (boxes) {
+      if (lane == 0) bulk_wait_group_read<0>();     // the stage below shares the area with the boxes
+      __syncwarp();
+    }
     if (a.gated) {
       const int c_first = chalf * (BN / 128), c_last = (chalf + 1) * (BN / 128);
-      __nv_bfloat16* act0 = act_out + row0 * ld_act;
-      __nv_bfloat16* pre0 = pre_out ? pre_out + row0 * ld_pre : nullptr;
-      if (rows_ok == 32 && t.n_tile * (BN / 2) + c_last * 32 <= a.N && ((ld_act | ld_pre | a.n_half) & 7) == 0 &&
-          aligned16(act0) && aligned16(pre0)) {
-        // Whole SwiGLU tile inside the matrix (the common case): the up half goes through the
-        // shared-memory stage first and is kept in the coalesced layout (4 lanes x 8 columns per
-        // row, 8 rows per pass), the gate half follows, and activation and both pre-activation
-        // halves are computed and stored in that layout: two trips through the stage per block
-        // instead of one per stored array.
-        const int sub = lane >> 2, c8 = (lane & 3) * 8;
-        float pr[4];
-#pragma unroll
-        for (int pass = 0; pass < 4; ++pass) pr[pass] = probs ? probs[row0 + pass * 8 + sub] : 1.0f;
-#pragma unroll 1
-        for (int c = c_first; c < c_last; ++c) {
-          const int col = t.n_tile * (BN / 2) + c * 32;
-          float ur[4][8];
-          {
-            float u[32];
-            load_acc(taddr + BN / 2 + c * 32, u, zero);
-            stage_put(stg, lane, u);
-          }
-#pragma unroll
-          for (int pass = 0; pass < 4; ++pass) {
-            const int rr = pass * 8 + sub;
-            const float4 xa = *reinterpret_cast<const float4*>(stg + rr * kStgLd + c8);
-            const float4 xb = *reinterpret_cast<const float4*>(stg + rr * kStgLd + c8 + 4);
-            ur[pass][0] = xa.x; ur[pass][1] = xa.y; ur[pass][2] = xa.z; ur[pass][3] = xa.w;
-            ur[pass][4] = xb.x; ur[pass][5] = xb.y; ur[pass][6] = xb.z; ur[pass][7] = xb.w;
-            if (pre0) {
-              uint4 q;
-              q.x = pack_bf16x2(xa.x, xa.y); q.y = pack_bf16x2(xa.z, xa.w);
-              q.z = pack_bf16x2(xb.x, xb.y); q.w = pack_bf16x2(xb.z, xb.w);
-              *reinterpret_cast<uint4*>(pre0 + (long long)rr * ld_pre + a.n_half + col + c8) = q;
-            }
-          }
-          {
-            float g[32];
-            load_acc(taddr + c * 32, g, zero);
-            stage_put(stg, lane, g);
-          }
-#pragma unroll
-          for (int pass = 0; pass < 4; ++pass) {
-            const int rr = pass * 8 + sub;
-            const float4 xa = *reinterpret_cast<const float4*>(stg + rr * kStgLd + c8);
-            const float4 xb = *reinterpret_cast<const float4*>(stg + rr * kStgLd + c8 + 4);
-            const float gv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-            if (pre0) {
-              uint4 q;
-              q.x = pack_bf16x2(xa.x, xa.y); q.y = pack_bf16x2(xa.z, xa.w);
-              q.z = pack_bf16x2(xb.x, xb.y); q.w = pack_bf16x2(xb.z, xb.w);
-              *reinterpret_cast<uint4*>(pre0 + (long long)rr * ld_pre + col + c8) = q;
-            }
-            float o[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = silu_f(gv[i]) * ur[pass][i] * pr[pass];
-            uint4 q;
-            q.x = pack_bf16x2(o[0], o[1]); q.y = pack_bf16x2(o[2], o[3]);
-            q.z = pack_bf16x2(o[4], o[5]); q.w = pack_bf16x2(o[6], o[7]);
-            *reinterpret_cast<uint4*>(act0 + (long long)rr * ld_act + col + c8) = q;
-          }
-        }
-        __syncwarp();
-        return;
-      }
 #pragma unroll 1
       for (int c = c_first; c < c_last; ++c) {
         const int col = t.n_tile * (BN / 2) + c * 32;
@@ -776,48 +790,6 @@ struct EpiAct {
       }
     } else {
       const int c_first = chalf * (BN / 64), c_last = (chalf + 1) * (BN / 64);
-      __nv_bfloat16* act0 = act_out + row0 * ld_act;
-      __nv_bfloat16* pre0 = pre_out ? pre_out + row0 * ld_pre : nullptr;
-      if (rows_ok == 32 && t.n_tile * BN + c_last * 32 <= a.N && ((ld_act | ld_pre) & 7) == 0 && aligned16(act0) &&
-          aligned16(pre0)) {
-        // Whole tile inside the matrix: one trip through the stage per block, pre-activation and
-        // activation are packed and stored from the coalesced layout.
-        const int sub = lane >> 2, c8 = (lane & 3) * 8;
-        float pr[4];
-#pragma unroll
-        for (int pass = 0; pass < 4; ++pass) pr[pass] = probs ? probs[row0 + pass * 8 + sub] : 1.0f;
-#pragma unroll 1
-        for (int c = c_first; c < c_last; ++c) {
-          const int col = t.n_tile * BN + c * 32;
-          {
-            float v[32];
-            load_acc(taddr + c * 32, v, zero);
-            stage_put(stg, lane, v);
-          }
-#pragma unroll
-          for (int pass = 0; pass < 4; ++pass) {
-            const int rr = pass * 8 + sub;
-            const float4 xa = *reinterpret_cast<const float4*>(stg + rr * kStgLd + c8);
-            const float4 xb = *reinterpret_cast<const float4*>(stg + rr * kStgLd + c8 + 4);
-            const float xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-            if (pre0) {
-              uint4 q;
-              q.x = pack_bf16x2(xa.x, xa.y); q.y = pack_bf16x2(xa.z, xa.w);
-              q.z = pack_bf16x2(xb.x, xb.y); q.w = pack_bf16x2(xb.z, xb.w);
-              *reinterpret_cast<uint4*>(pre0 + (long long)rr * ld_pre + col + c8) = q;
-            }
-            float o[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = act_f(act_kind, xv[i]) * pr[pass];
-            uint4 q;
-            q.x = pack_bf16x2(o[0], o[1]); q.y = pack_bf16x2(o[2], o[3]);
-            q.z = pack_bf16x2(o[4], o[5]); q.w = pack_bf16x2(o[6], o[7]);
-            *reinterpret_cast<uint4*>(act0 + (long long)rr * ld_act + col + c8) = q;
-          }
-        }
-        __syncwarp();
-        return;
-      }
 #pragma unroll 1
       for (int c = c_first; c < c_last; ++c) {
         const int col = t.n_tile * BN + c * 32;
@@ -855,6 +827,42 @@ struct EpiDAct {
   int act_kind;
   int gated;   // activation is SwiGLU: pre_in / dpre hold [gate | up] halves `n_half` apart
   int n_half;
+  int boxes;   // pre-activation (map 0) and its gradient (map 1) can be moved by bulk tensor copies
+
+  // Whole blocks: boxes of 32 rows x 32 columns of the pre-activation (gate and up) are copied in, turned
+  // into the gradient in place one row per lane, which is the accumulator's own layout, and copied out.  Two
+  // sets of boxes alternate, as in the optimizer epilogue.
+  // Against loads and stores from registers around a trip of the accumulator through shared memory:
+  // SwiGLU 8 x 1024 rows, 4096 -> 14336, 0.80 -> 0.78 ms; 64 x 768 rows, 2048 -> 1408, 316 -> 292 us; GELU 64 x
+  // 1024 rows, 2048 -> 1024, 300 -> 269 us (437 with the error function evaluated twice).
+  static constexpr int kBox = 32 * 64;
+  static constexpr int kWarpBytes = 2 * 2 * kBox;
+  template <int BN>
+  __device__ __forceinline__ bool whole(const Tile& t, const GemmArgs& a, int r, int chalf) const {
+    // four blocks a tile (BN 256): each set is filled twice, so its barrier's phase starts every tile at 0
+    return BN == 256 && boxes && t.rows_valid - (r & ~31) >= 32 && t.n_tile * BN + (chalf + 1) * (BN / 2) <= a.N;
+  }
+  __device__ __forceinline__ void load_set(const CUtensorMap* maps, uint8_t* set, uint64_t* bar, int col,
+                                           int row) const {
+    const int n = gated ? 2 : 1;
+    mbar_expect_tx(bar, n * kBox);
+    for (int i = 0; i < n; ++i) tma_load_3d(set + i * kBox, maps, bar, col + i * n_half, row, 0);
+  }
+  template <int BN>
+  __device__ __forceinline__ void fetch(const Tile& t, const GemmArgs& a, int r, int chalf, float* stg,
+                                        const CUtensorMap* maps, uint64_t* wbar) const {
+    if (!whole<BN>(t, a, r, chalf)) return;
+    fence_proxy_async_smem();         // what this warp stored in its area by other means is done
+    __syncwarp();
+    if ((r & 31) == 0) {
+      bulk_wait_group_read<0>();      // the last tile's boxes have left
+      const int col = t.n_tile * BN + chalf * (BN / 2);
+      uint8_t* sets = reinterpret_cast<uint8_t*>(stg);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) load_set(maps, sets + i * 2 * kBox, wbar + i, col + 32 * i, t.row_base + t.m0 + r);
+    }
+    __syncwarp();
+  }
 
   static constexpr bool kPrefetch = true;
   // Called one tile ahead: pull this thread's row of the pre-activations (gate and up half of the
@@ -884,136 +892,86 @@ struct EpiDAct {
     const float p = (row_ok && probs) ? probs[row] : 1.0f;
     float dp = 0.f;
     const int c_first = chalf * (BN / 64), c_last = (chalf + 1) * (BN / 64);
-    const __nv_bfloat16* pre0 = pre_in + row0 * ld_pre_in;
-    __nv_bfloat16* dpre0 = dpre + row0 * ld_dpre;
-    if (gated && rows_ok == 32 && t.n_tile * BN + c_last * 32 <= a.N && ((ld_pre_in | ld_dpre | n_half) & 7) == 0 &&
-        aligned16(pre0) && aligned16(dpre0)) {
-      // Whole SwiGLU tile inside the matrix (the common case).  Only the accumulator goes through
-      // the shared-memory stage; gate and up pre-activations are read, and their gradients written,
-      // in the coalesced layout (4 lanes x 16 bytes per row, 8 rows per pass), and all eight loads
-      // of a block are issued before the accumulator is fetched, so their latency overlaps.  The
-      // probability gradient is summed per (row, lane quad) and folded to one value per row at the end.
-      const int sub = lane >> 2, c8 = (lane & 3) * 8;
-      float pr[4], dq[4];
-#pragma unroll
-      for (int pass = 0; pass < 4; ++pass) {
-        pr[pass] = probs ? probs[row0 + pass * 8 + sub] : 1.0f;
-        dq[pass] = 0.f;
-      }
+    if (whole<BN>(t, a, r, chalf)) {
+      uint8_t* const sets = reinterpret_cast<uint8_t*>(stg);
+      const int swz = (lane >> 1) & 3;
+      const int boxes_of_set = gated ? 2 : 1;
+      float d4[4] = {0.f, 0.f, 0.f, 0.f};      // four partial sums of the row
 #pragma unroll 1
-      for (int c = c_first; c < c_last; ++c) {
-        const int col = t.n_tile * BN + c * 32;
-        uint4 rg[4], ru[4];
-#pragma unroll
-        for (int pass = 0; pass < 4; ++pass) {
-          const long long o = (long long)(pass * 8 + sub) * ld_pre_in + col + c8;
-          rg[pass] = *reinterpret_cast<const uint4*>(pre0 + o);
-          ru[pass] = *reinterpret_cast<const uint4*>(pre0 + o + n_half);
+      for (int k = 0; k < BN / 64; ++k) {
+        const int col = t.n_tile * BN + (c_first + k) * 32;
+        uint8_t* const set = sets + (k & 1) * 2 * kBox;
+        float v[32];
+        load_acc(taddr + (c_first + k) * 32, v, zero);
+        if (lane == 0 && k > 0 && k + 1 < BN / 64) {
+          // the set of the block before has left: refill it for the block after this one
+          bulk_wait_group_read<0>();
+          load_set(maps, sets + ((k + 1) & 1) * 2 * kBox, wbar + ((k + 1) & 1), col + 32, (int)row0);
         }
-        {
-          float v[32];
-          load_acc(taddr + c * 32, v, zero);
-          stage_put(stg, lane, v);
+        __syncwarp();
+        if (!mbar_wait(wbar + (k & 1), (k >> 1) & 1, a.timeout_ns, abort_flag)) {
+          if (lane == 0) report_status(a.status, kStatusMbarTimeout, kKernelIdGemm2, 510 + k, 0, 0);
+          return;
         }
 #pragma unroll
-        for (int pass = 0; pass < 4; ++pass) {
-          const int rr = pass * 8 + sub;
-          const float4 va = *reinterpret_cast<const float4*>(stg + rr * kStgLd + c8);
-          const float4 vb = *reinterpret_cast<const float4*>(stg + rr * kStgLd + c8 + 4);
-          const float vv[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
-          const uint32_t* wg = reinterpret_cast<const uint32_t*>(&rg[pass]);
-          const uint32_t* wu = reinterpret_cast<const uint32_t*>(&ru[pass]);
+        for (int j = 0; j < 4; ++j) {
+          uint4* const at = reinterpret_cast<uint4*>(set + lane * 64 + ((j ^ swz) << 4));
+          const uint4 rg = at[0];
+          const uint32_t wg[4] = {rg.x, rg.y, rg.z, rg.w};
           float og[8], ou[8];
+          if (gated) {
+            const uint4 ru = at[kBox / 16];
+            const uint32_t wu[4] = {ru.x, ru.y, ru.z, ru.w};
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            // bf16 -> fp32 is a 16-bit shift of the bit pattern
-            const uint32_t gw = wg[i >> 1], uw = wu[i >> 1];
-            const float gi = __uint_as_float((i & 1) ? (gw & 0xffff0000u) : (gw << 16));
-            const float ui = __uint_as_float((i & 1) ? (uw & 0xffff0000u) : (uw << 16));
-            const float sg = sigmoid_f(gi);
-            const float sl = gi * sg;
-            dq[pass] += vv[i] * sl * ui;
-            const float da = vv[i] * pr[pass];
-            og[i] = da * ui * (sg * (1.0f + gi * (1.0f - sg)));
-            ou[i] = da * sl;
+            for (int i = 0; i < 8; ++i) {
+              // bf16 -> fp32 is a 16-bit shift of the bit pattern
+              const float gi = __uint_as_float((i & 1) ? (wg[i >> 1] & 0xffff0000u) : (wg[i >> 1] << 16));
+              const float ui = __uint_as_float((i & 1) ? (wu[i >> 1] & 0xffff0000u) : (wu[i >> 1] << 16));
+              const float x = v[8 * j + i];
+              const float sg = sigmoid_f(gi);          // one sigmoid serves silu and its derivative
+              const float sl = gi * sg;
+              d4[i & 3] += x * sl * ui;
+              const float da = x * p;
+              og[i] = da * ui * (sg * (1.0f + gi * (1.0f - sg)));
+              ou[i] = da * sl;
+            }
+            at[kBox / 16] = make_uint4(pack_bf16x2(ou[0], ou[1]), pack_bf16x2(ou[2], ou[3]), pack_bf16x2(ou[4], ou[5]),
+                                       pack_bf16x2(ou[6], ou[7]));
+          } else {
+            auto plain = [&](auto kind) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const float xi = __uint_as_float((i & 1) ? (wg[i >> 1] & 0xffff0000u) : (wg[i >> 1] << 16));
+                const float x = v[8 * j + i];
+                float y, dy;
+                act_dact<decltype(kind)::value>(xi, y, dy);
+                d4[i & 3] += x * y;
+                og[i] = x * p * dy;
+              }
+            };
+            if (act_kind == FM_ACT_GELU) plain(Kind<FM_ACT_GELU>{});
+            else if (act_kind == FM_ACT_SILU) plain(Kind<FM_ACT_SILU>{});
+            else plain(Kind<FM_ACT_NONE>{});
           }
-          uint4 pg, pu;
-          pg.x = pack_bf16x2(og[0], og[1]); pg.y = pack_bf16x2(og[2], og[3]);
-          pg.z = pack_bf16x2(og[4], og[5]); pg.w = pack_bf16x2(og[6], og[7]);
-          pu.x = pack_bf16x2(ou[0], ou[1]); pu.y = pack_bf16x2(ou[2], ou[3]);
-          pu.z = pack_bf16x2(ou[4], ou[5]); pu.w = pack_bf16x2(ou[6], ou[7]);
-          const long long o = (long long)rr * ld_dpre + col + c8;
-          *reinterpret_cast<uint4*>(dpre0 + o) = pg;
-          *reinterpret_cast<uint4*>(dpre0 + o + n_half) = pu;
+          at[0] = make_uint4(pack_bf16x2(og[0], og[1]), pack_bf16x2(og[2], og[3]), pack_bf16x2(og[4], og[5]),
+                             pack_bf16x2(og[6], og[7]));
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          for (int i = 0; i < boxes_of_set; ++i)
+            tma_store_3d(maps + 1, set + i * kBox, col + i * n_half, (int)row0, 0);
+          bulk_commit_group();
         }
       }
       __syncwarp();
-      // row pass * 8 + sub: sum over its four lanes, then hand every lane the sum of its own row
-#pragma unroll
-      for (int pass = 0; pass < 4; ++pass) {
-        float x = dq[pass];
-        x += __shfl_xor_sync(0xffffffffu, x, 1);
-        x += __shfl_xor_sync(0xffffffffu, x, 2);
-        x = __shfl_sync(0xffffffffu, x, (lane & 7) * 4);
-        if ((lane >> 3) == pass) dp = x;
-      }
+      dp = (d4[0] + d4[1]) + (d4[2] + d4[3]);
       if (dprobs_partial) dprobs_partial[(row * n_tiles + t.n_tile) * 2 + chalf] = dp;
       return;
     }
-    if (!gated && rows_ok == 32 && t.n_tile * BN + c_last * 32 <= a.N && ((ld_pre_in | ld_dpre) & 7) == 0 &&
-        aligned16(pre0) && aligned16(dpre0)) {
-      // The same for a plain activation (GELU, SiLU): one array in, one out.
-      const int sub = lane >> 2, c8 = (lane & 3) * 8;
-      float pr[4], dq[4];
-#pragma unroll
-      for (int pass = 0; pass < 4; ++pass) {
-        pr[pass] = probs ? probs[row0 + pass * 8 + sub] : 1.0f;
-        dq[pass] = 0.f;
-      }
-#pragma unroll 1
-      for (int c = c_first; c < c_last; ++c) {
-        const int col = t.n_tile * BN + c * 32;
-        uint4 rx[4];
-#pragma unroll
-        for (int pass = 0; pass < 4; ++pass)
-          rx[pass] = *reinterpret_cast<const uint4*>(pre0 + (long long)(pass * 8 + sub) * ld_pre_in + col + c8);
-        {
-          float v[32];
-          load_acc(taddr + c * 32, v, zero);
-          stage_put(stg, lane, v);
-        }
-#pragma unroll
-        for (int pass = 0; pass < 4; ++pass) {
-          const int rr = pass * 8 + sub;
-          const float4 va = *reinterpret_cast<const float4*>(stg + rr * kStgLd + c8);
-          const float4 vb = *reinterpret_cast<const float4*>(stg + rr * kStgLd + c8 + 4);
-          const float vv[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
-          const uint32_t* wx = reinterpret_cast<const uint32_t*>(&rx[pass]);
-          float o[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const uint32_t xw = wx[i >> 1];
-            const float xi = __uint_as_float((i & 1) ? (xw & 0xffff0000u) : (xw << 16));
-            dq[pass] += vv[i] * act_f(act_kind, xi);
-            o[i] = vv[i] * pr[pass] * dact_f(act_kind, xi);
-          }
-          uint4 q;
-          q.x = pack_bf16x2(o[0], o[1]); q.y = pack_bf16x2(o[2], o[3]);
-          q.z = pack_bf16x2(o[4], o[5]); q.w = pack_bf16x2(o[6], o[7]);
-          *reinterpret_cast<uint4*>(dpre0 + (long long)rr * ld_dpre + col + c8) = q;
-        }
-      }
+    if (boxes) {
+      if (lane == 0) bulk_wait_group_read<0>();     // the stage below shares the area with the boxes
       __syncwarp();
-#pragma unroll
-      for (int pass = 0; pass < 4; ++pass) {
-        float x = dq[pass];
-        x += __shfl_xor_sync(0xffffffffu, x, 1);
-        x += __shfl_xor_sync(0xffffffffu, x, 2);
-        x = __shfl_sync(0xffffffffu, x, (lane & 7) * 4);
-        if ((lane >> 3) == pass) dp = x;
-      }
-      if (dprobs_partial) dprobs_partial[(row * n_tiles + t.n_tile) * 2 + chalf] = dp;
-      return;
     }
 #pragma unroll 1
     for (int c = c_first; c < c_last; ++c) {
@@ -1599,14 +1557,25 @@ extern "C" int fm_gemm_launch(const FmGemmDesc* d, cudaStream_t stream) {
     }
     case FM_EPI_ACT: {
       EpiAct e{reinterpret_cast<__nv_bfloat16*>(d->act_out), d->ld_act,
-               reinterpret_cast<__nv_bfloat16*>(d->pre_out), d->ld_pre, d->probs, d->act_kind};
+               reinterpret_cast<__nv_bfloat16*>(d->pre_out), d->ld_pre, d->probs, d->act_kind, 0};
+      const long long rows = d->a_mn ? d->a_inner : d->a_outer;
+      // a copy starts on 16 bytes: the up half at a multiple of 8 columns
+      e.boxes = (!d->gated || d->n_half % 8 == 0) &&
+                make_out_map(&maps.m[1], d->act_out, false, d->N, rows, d->ld_act, 1, 0) &&
+                (d->pre_out == nullptr ||
+                 make_out_map(&maps.m[0], d->pre_out, false, d->gated ? d->n_half + d->N : d->N, rows, d->ld_pre, 1, 0));
       return dispatch_gate(d, ta, tb, args, e, maps, grid, stream);
     }
     case FM_EPI_DACT: {
       const int nt = (d->N + d->bn - 1) / d->bn;
       EpiDAct e{reinterpret_cast<const __nv_bfloat16*>(d->pre_in), d->ld_pre_in,
                 reinterpret_cast<__nv_bfloat16*>(d->C), d->ldc, d->probs, d->dprobs, nt,
-                d->act_kind, d->gated, d->n_half};
+                d->act_kind, d->gated, d->n_half, 0};
+      const long long rows = d->a_mn ? d->a_inner : d->a_outer, cols = d->gated ? d->n_half + d->N : d->N;
+      // a copy starts on 16 bytes: the up half at a multiple of 8 columns
+      e.boxes = (!d->gated || d->n_half % 8 == 0) &&
+                make_out_map(&maps.m[0], d->pre_in, false, cols, rows, d->ld_pre_in, 1, 0, 64) &&
+                make_out_map(&maps.m[1], d->C, false, cols, rows, d->ldc, 1, 0, 64);
       args.gated = 0;  // here `gated` describes the activation, not the layout of B
       return dispatch_gate(d, ta, tb, args, e, maps, grid, stream);
     }

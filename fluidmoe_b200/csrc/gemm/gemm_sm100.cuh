@@ -292,7 +292,7 @@ struct GateKSource {
 
 template <int BN, class Epi>
 constexpr int gemm_stages() {
-  return EpiStaging<Epi>::fetches ? (BN == 256 ? 2 : 3) : (BN == 256 ? 3 : 4);
+  return (BN == 256 ? 3 : 4) - (EpiStaging<Epi>::bytes > 4 * kEpiStageFloats ? 1 : 0);
 }
 template <int BN, class Epi>
 constexpr int gemm_smem_bytes() {
@@ -579,7 +579,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
 // =========================================================================================
 template <class Epi>
 constexpr int gemm2_stages() {
-  return EpiStaging<Epi>::fetches ? 4 : 5;
+  return EpiStaging<Epi>::bytes > 4 * kEpiStageFloats ? 4 : 5;
 }
 template <class Epi>
 constexpr int gemm2_smem_bytes() {

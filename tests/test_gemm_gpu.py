@@ -344,3 +344,53 @@ def test_wgrad_adam_in_boxes_agrees_with_the_path_through_registers(G, rows, M, 
     for s, box, reg in zip(start, *results):
         assert not torch.equal(s, box)
         torch.testing.assert_close(box.float(), reg.float(), rtol=2.0 ** -7, atol=1e-6)
+
+
+@pytest.mark.parametrize("act", ["gelu", "silu", "swiglu"])
+@pytest.mark.parametrize("rows,F", [([64, 33, 0, 31], 264), ([32, 96, 1, 256], 512), ([300, 20, 64, 64], 128)])
+@pytest.mark.parametrize("cta_pair", [0, 1])
+@pytest.mark.parametrize("lead", [0, 1])
+def test_activation_epilogues_at_ragged_groups_and_edges(act, rows, F, cta_pair, lead, monkeypatch):
+    """FC1 and the FC2 input gradient: whole blocks move in boxes, the rest and bases off 16 bytes (`lead`)
+    through registers; rows of no group stay as they were."""
+    monkeypatch.setattr(gemm, "CTA_PAIR", cta_pair)
+    torch.manual_seed(F)
+    if act == "swiglu" and F <= 128:
+        F = 136          # gated tiles are 256 wide
+    G, H = len(rows), 128
+    offs = [sum(rows[:g]) for g in range(G)]
+    total = sum(rows) + 40
+    Fw = 2 * F if act == "swiglu" else F
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
+
+    def fresh(n):
+        return torch.full((total * n + 8,), 7.0, dtype=torch.bfloat16, device="cuda")[lead:lead + total * n].view(total, n)
+
+    x, w1, w2 = _rand(total, H), _rand(G, H, Fw, scale=0.1), _rand(G, F, H, scale=0.1)
+    probs, dy = torch.rand(total, device="cuda"), _rand(total, H)
+    kw = dict(activation=act, group_rows=i32(rows), group_offs=i32(offs))
+    a, pre = gemm.grouped_gemm_act(x, w1, probs, act_out=fresh(F), pre_out=fresh(Fw), **kw)
+    a2, none = gemm.grouped_gemm_act(x, w1, probs, act_out=fresh(F), save_pre=False, **kw)
+    dpre, dprobs = gemm.grouped_gemm_dact(dy, w2, pre, probs, dpre_out=fresh(Fw), **kw)
+    torch.cuda.synchronize()
+    gemm.check_status()
+    assert none is None and torch.equal(a, a2)
+    for t in (a, pre, dpre):
+        assert (t[sum(rows):] == 7.0).all()
+    for g in range(G):
+        r = slice(offs[g], offs[g] + rows[g])
+        p = probs[r].double()[:, None]
+        ref_pre = x[r].double() @ w1[g].double()
+        # one rounding of bf16 (2^-8) after fp32 sums and fast exponentials
+        def close(got, ref, rel=2.0 ** -8, floor=2e-4):
+            assert ((got.double() - ref).abs() <= rel * ref.abs() + floor * ref.abs().max().clamp(min=1e-9)).all()
+        if rows[g] == 0:
+            continue
+        close(pre[r], ref_pre)
+        close(a[r], gemm.act_ref(ref_pre, act) * p)
+        z = pre[r].double().requires_grad_(True)
+        y = gemm.act_ref(z, act)
+        d = dy[r].double() @ w2[g].double().t()
+        (dz,) = torch.autograd.grad(y, z, d * p)
+        close(dpre[r], dz)
+        close(dprobs[r], (d * y.detach()).sum(1), rel=1e-5)
