@@ -120,66 +120,113 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 // --------------------------------------------------------------------------------------------
 // Normalisation backward.  Each CTA walks rows blockIdx.x, +gridDim.x, ...; a thread owns the
 // same columns in every row, so the weight / bias gradients accumulate in registers and are
-// written once per CTA to a partial buffer [gridDim.x, 2, H] that a second kernel reduces.
-// dx optionally adds the gradient that reaches the input through the residual branch.
+// written once per CTA to a partial buffer [gridDim.x, 2, H] (RMSNorm: [gridDim.x, H]) that a second
+// kernel reduces.  dx optionally adds the gradient that reaches the input through the residual branch.
+// Bound by memory (8 bytes an element with the residual): the loads of the next row are issued before the
+// one barrier of the current row, both sums cross it together, and what the second half needs is
+// unpacked again from the 16-byte words instead of being kept.  With the reduction, residual included: RMSNorm
+// 4096 x 4096 (134 MB) 85 -> 36 us, 8192 x 2048 75 -> 38 us, LayerNorm 2048 x 1024 30 -> 15 us.
 // --------------------------------------------------------------------------------------------
 constexpr int kNormBwdChunks = 4;  // columns per thread = 8 * chunks  ->  H <= 8192
+constexpr int kNormBwdBlocks = 2 * 148;
 
-// kChunks (1, 2 or 4) is chosen from H: the per-thread arrays below are sized by it, and with
-// four chunks the kernel needs 195 registers, which leaves one CTA of eight warps per SM and makes
-// it latency-bound (0.31 of the copy bandwidth at H = 4096); two chunks fit two CTAs per SM.
-template <int kChunks>
+// kChunks (1, 2 or 4) is chosen from H: the per-thread arrays below are sized by it; one or two chunks fit
+// two CTAs per SM.
+template <int kChunks, bool kLayerNorm>
 __global__ void __launch_bounds__(kNormThreads, kChunks <= 2 ? 2 : 1)
 norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                 const __nv_bfloat16* __restrict__ w, const float* __restrict__ mean,
                 const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ res_grad,
-                __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int T, int H,
-                int kind) {
-  __shared__ float red[kNormThreads / 32];
-  const int nvec = H / 8;
-  float dg[kChunks][8], db[kChunks][8], g[kChunks][8];
+                __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int T, int H) {
+  constexpr int kWarps = kNormThreads / 32;
+  __shared__ float2 red[2][kWarps];
+  const int nvec = H / 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float dg[kChunks][8], db[kLayerNorm ? kChunks : 1][8];
+  uint4 pw[kChunks];
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
     const int i = threadIdx.x + c * kNormThreads;
-    if (i < nvec) unpack8(reinterpret_cast<const uint4*>(w)[i], g[c]);
+    pw[c] = i < nvec ? reinterpret_cast<const uint4*>(w)[i] : make_uint4(0, 0, 0, 0);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) dg[c][j] = db[c][j] = 0.f;
+    for (int j = 0; j < 8; ++j) {
+      dg[c][j] = 0.f;
+      if (kLayerNorm) db[c][j] = 0.f;
+    }
   }
-  for (long long r = blockIdx.x; r < T; r += gridDim.x) {
-    const float mu = kind == 0 ? mean[r] : 0.f;
-    const float rs = rstd[r];
-    float xh[kChunks][8], gy[kChunks][8];
-    float s1 = 0.f, s2 = 0.f;
+  uint4 px[kChunks], pd[kChunks], pr[kChunks];
+  float mu = 0.f, rs = 0.f;
+  auto fetch = [&](long long r) {
+    if (kLayerNorm) mu = mean[r];
+    rs = rstd[r];
 #pragma unroll
     for (int c = 0; c < kChunks; ++c) {
       const int i = threadIdx.x + c * kNormThreads;
+      px[c] = pd[c] = pr[c] = make_uint4(0, 0, 0, 0);
       if (i < nvec) {
-        float xv[8], dv[8];
-        unpack8(reinterpret_cast<const uint4*>(x + r * H)[i], xv);
-        unpack8(reinterpret_cast<const uint4*>(dy + r * H)[i], dv);
+        px[c] = reinterpret_cast<const uint4*>(x + r * H)[i];
+        pd[c] = reinterpret_cast<const uint4*>(dy + r * H)[i];
+        if (res_grad != nullptr) pr[c] = reinterpret_cast<const uint4*>(res_grad + r * H)[i];
+      }
+    }
+  };
+  int buf = 0;
+  if (blockIdx.x < T) fetch(blockIdx.x);
+  for (long long r = blockIdx.x; r < T; r += gridDim.x, buf ^= 1) {
+    uint4 cx[kChunks], cd[kChunks], cr[kChunks];
+    const float cmu = mu, crs = rs;
+    float2 s = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          xh[c][j] = (xv[j] - mu) * rs;
-          gy[c][j] = dv[j] * g[c][j];
-          s1 += gy[c][j] * xh[c][j];
-          s2 += gy[c][j];
-          dg[c][j] += dv[j] * xh[c][j];
-          db[c][j] += dv[j];
+    for (int c = 0; c < kChunks; ++c) {
+      cx[c] = px[c];
+      cd[c] = pd[c];
+      cr[c] = pr[c];
+      float xv[8], dv[8], gv[8];
+      unpack8(cx[c], xv);
+      unpack8(cd[c], dv);
+      unpack8(pw[c], gv);
+      const bool in = threadIdx.x + c * kNormThreads < nvec;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float xh = (xv[j] - cmu) * crs;
+        const float gy = dv[j] * gv[j];
+        s.x += gy * xh;
+        s.y += gy;
+        if (in) {
+          dg[c][j] += dv[j] * xh;
+          if (kLayerNorm) db[c][j] += dv[j];
         }
       }
     }
-    const float c1 = block_sum<kNormThreads>(s1, red) / H;
-    const float c2 = kind == 0 ? block_sum<kNormThreads>(s2, red) / H : 0.f;
+    if (r + gridDim.x < T) fetch(r + gridDim.x);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+      if (kLayerNorm) s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    if (lane == 0) red[buf][warp] = s;      // two buffers: one barrier a row
+    __syncthreads();
+    float c1 = 0.f, c2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < kWarps; ++i) {
+      const float2 t = red[buf][i];
+      c1 += t.x;
+      c2 += t.y;
+    }
+    c1 /= H;
+    c2 = kLayerNorm ? c2 / H : 0.f;
 #pragma unroll
     for (int c = 0; c < kChunks; ++c) {
       const int i = threadIdx.x + c * kNormThreads;
       if (i < nvec) {
-        float o[8];
+        float xv[8], dv[8], gv[8], o[8];
+        unpack8(cx[c], xv);
+        unpack8(cd[c], dv);
+        unpack8(pw[c], gv);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = (gy[c][j] - c2 - xh[c][j] * c1) * rs;
+        for (int j = 0; j < 8; ++j) o[j] = (dv[j] * gv[j] - c2 - (xv[j] - cmu) * crs * c1) * crs;
         if (res_grad != nullptr) {
           float rg[8];
-          unpack8(reinterpret_cast<const uint4*>(res_grad + r * H)[i], rg);
+          unpack8(cr[c], rg);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += rg[j];
         }
@@ -187,40 +234,46 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
       }
     }
   }
-  float* pg = partial + (long long)blockIdx.x * 2 * H;
+  float* pg = partial + (long long)blockIdx.x * (kLayerNorm ? 2 : 1) * H;
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
     const int i = threadIdx.x + c * kNormThreads;
     if (i < nvec) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        pg[i * 8 + j] = dg[c][j];
-        pg[H + i * 8 + j] = db[c][j];
+      *reinterpret_cast<float4*>(pg + i * 8) = make_float4(dg[c][0], dg[c][1], dg[c][2], dg[c][3]);
+      *reinterpret_cast<float4*>(pg + i * 8 + 4) = make_float4(dg[c][4], dg[c][5], dg[c][6], dg[c][7]);
+      if (kLayerNorm) {
+        *reinterpret_cast<float4*>(pg + H + i * 8) = make_float4(db[c][0], db[c][1], db[c][2], db[c][3]);
+        *reinterpret_cast<float4*>(pg + H + i * 8 + 4) = make_float4(db[c][4], db[c][5], db[c][6], db[c][7]);
       }
     }
   }
 }
 
-// Column sums of the partial buffer: a CTA owns 32 columns, its eight warps take every eighth
-// partial row each and the eight sums meet in shared memory.
-__global__ void __launch_bounds__(256)
+// Column sums of the partial buffer [nblocks][cols]: a CTA owns 32 columns, its 32 warps take every 32nd
+// partial row each and the sums meet in shared memory.
+__global__ void __launch_bounds__(1024)
 norm_bwd_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw,
-                       float* __restrict__ db, int nblocks, int H) {
-  __shared__ float part[8][33];
+                       float* __restrict__ db, int nblocks, int cols, int H) {
+  __shared__ float part[32][33];
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + lane;
   float s = 0.f;
-  if (col < 2 * H)
-    for (int b = grp; b < nblocks; b += 8) s += partial[(long long)b * 2 * H + col];
+  if (col < cols) {
+#pragma unroll 4
+    for (int b = grp; b < nblocks; b += 32) s += partial[(long long)b * cols + col];
+  }
   part[grp][lane] = s;
   __syncthreads();
-  if (grp == 0 && col < 2 * H) {
+  // column `grp` of the CTA: one partial sum per lane
+  s = part[lane][grp];
 #pragma unroll
-    for (int g2 = 1; g2 < 8; ++g2) s += part[g2][lane];
-    if (col < H)
-      dw[col] = s;
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  const int c = blockIdx.x * 32 + grp;
+  if (lane == 0 && c < cols) {
+    if (c < H)
+      dw[c] = s;
     else if (db != nullptr)
-      db[col - H] = s;
+      db[c - H] = s;
   }
 }
 
@@ -309,39 +362,43 @@ constexpr int kKernelIdUnpermuteWait = 15;
 // have reached `wait_expected` (rows pushed by peers into `rows`): the consumer polls its own
 // counters instead of a stand-alone wait kernel in front of it.  The time the slowest thread of CTA 0
 // waited is added to `wait_ns` (communication the step could not hide).
-__global__ void unpermute_reduce_kernel(const __nv_bfloat16* __restrict__ rows,
-                                        const int* __restrict__ slot,
-                                        const __nv_bfloat16* __restrict__ residual,
-                                        __nv_bfloat16* __restrict__ out, int T, int k, int H,
-                                        const int* wait_flags, int wait_n, int wait_expected,
-                                        unsigned long long* wait_ns, unsigned long long timeout_ns,
-                                        int* status) {
+// One thread per 16 bytes of a token, K known at compile time: the k rows and the residual are in flight
+// together, and a few tokens still fill the chip.  With one warp per token and a loop over k, 8192 tokens of
+// 2048 columns and k = 8 (336 MB) took 99 us, now 57; 64 tokens of 4096 columns and k = 2 17 us, now 6.
+template <int K>
+__global__ void __launch_bounds__(256)
+unpermute_reduce_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict__ slot,
+                        const __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ out, int T, int k,
+                        int H, const int* wait_flags, int wait_n, int wait_expected, unsigned long long* wait_ns,
+                        unsigned long long timeout_ns, int* status) {
   if (wait_flags != nullptr)
     wait_counters_cta(wait_flags, wait_n, wait_expected, wait_ns, timeout_ns, status, kKernelIdUnpermuteWait);
-  const int nvec = H / 8;
-  const int warps_per_block = blockDim.x >> 5;
-  const int lane = threadIdx.x & 31;
-  for (long long t = (long long)blockIdx.x * warps_per_block + (threadIdx.x >> 5); t < T;
-       t += (long long)gridDim.x * warps_per_block) {
-    int sl[16];
-    for (int j = 0; j < k; ++j) sl[j] = slot[t * k + j];
-    for (int i = lane; i < nvec; i += 32) {
-      float acc[8];
-      if (residual != nullptr) {
-        unpack8(reinterpret_cast<const uint4*>(residual + t * H)[i], acc);
-      } else {
+  const unsigned nvec = H / 8;
+  const long long total = (long long)T * nvec;
+  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
+       idx += (long long)gridDim.x * blockDim.x) {
+    const long long t = total <= 0xffffffffll ? (long long)((unsigned)idx / nvec) : idx / nvec;
+    const int i = (int)(idx - t * nvec);
+    uint4 v[K];
+    int sl[K];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) acc[q] = 0.f;
-      }
-      for (int j = 0; j < k; ++j) {
-        if (sl[j] < 0) continue;
-        float v[8];
-        unpack8(reinterpret_cast<const uint4*>(rows + (long long)sl[j] * H)[i], v);
+    for (int j = 0; j < K; ++j) sl[j] = j < k ? slot[t * k + j] : -1;
+    uint4 res = make_uint4(0, 0, 0, 0);
+    if (residual != nullptr) res = reinterpret_cast<const uint4*>(residual + t * H)[i];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) acc[q] += v[q];
-      }
-      reinterpret_cast<uint4*>(out + t * H)[i] = pack8(acc);
+    for (int j = 0; j < K; ++j)
+      if (sl[j] >= 0) v[j] = reinterpret_cast<const uint4*>(rows + (long long)sl[j] * H)[i];
+    float acc[8];
+    unpack8(res, acc);
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      if (sl[j] < 0) continue;
+      float x[8];
+      unpack8(v[j], x);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[q] += x[q];
     }
+    reinterpret_cast<uint4*>(out + t * H)[i] = pack8(acc);
   }
 }
 
@@ -637,7 +694,7 @@ extern "C" int fm_norm_fwd(const void* x, const void* w, const void* b, void* y,
   return check_launch("norm_fwd");
 }
 
-extern "C" int fm_norm_bwd_blocks(int T) { return T < 592 ? T : 592; }
+extern "C" int fm_norm_bwd_blocks(int T) { return T < fm::kNormBwdBlocks ? T : fm::kNormBwdBlocks; }
 
 extern "C" int fm_norm_bwd(const void* dy, const void* x, const void* w, const float* mean,
                            const float* rstd, const void* res_grad, void* dx, float* partial,
@@ -649,16 +706,18 @@ extern "C" int fm_norm_bwd(const void* dy, const void* x, const void* w, const f
   using bf = __nv_bfloat16;
   const int nb = fm_norm_bwd_blocks(T);
   const int nvec = H / 8;
-  auto launch = [&](auto kernel) {
+  auto launch = [&](auto layer_norm, auto rms_norm) {
+    auto kernel = kind == 0 ? layer_norm : rms_norm;
     kernel<<<nb, fm::kNormThreads, 0, s>>>((const bf*)dy, (const bf*)x, (const bf*)w, mean, rstd,
-                                           (const bf*)res_grad, (bf*)dx, partial, T, H, kind);
+                                           (const bf*)res_grad, (bf*)dx, partial, T, H);
   };
-  if (nvec <= fm::kNormThreads) launch(fm::norm_bwd_kernel<1>);
-  else if (nvec <= 2 * fm::kNormThreads) launch(fm::norm_bwd_kernel<2>);
-  else launch(fm::norm_bwd_kernel<4>);
+  if (nvec <= fm::kNormThreads) launch(fm::norm_bwd_kernel<1, true>, fm::norm_bwd_kernel<1, false>);
+  else if (nvec <= 2 * fm::kNormThreads) launch(fm::norm_bwd_kernel<2, true>, fm::norm_bwd_kernel<2, false>);
+  else launch(fm::norm_bwd_kernel<4, true>, fm::norm_bwd_kernel<4, false>);
   int rc = check_launch("norm_bwd");
   if (rc) return rc;
-  fm::norm_bwd_reduce_kernel<<<(2 * H + 31) / 32, 256, 0, s>>>(partial, dw, db, nb, H);
+  const int cols = kind == 0 ? 2 * H : H;
+  fm::norm_bwd_reduce_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(partial, dw, db, nb, cols, H);
   return check_launch("norm_bwd_reduce");
 }
 
@@ -702,14 +761,7 @@ extern "C" int fm_gather_rows(const void* x, const long long* idx, void* out, lo
 
 extern "C" int fm_unpermute_reduce(const void* rows, const int* slot, const void* residual,
                                    void* out, int T, int k, int H, cudaStream_t s) {
-  if (H % 8 != 0 || k > 16) {
-    fm_set_error("unpermute_reduce: H must be a multiple of 8 and k at most 16");
-    return -1;
-  }
-  fm::unpermute_reduce_kernel<<<grid_for(T, 8), 256, 0, s>>>(
-      (const __nv_bfloat16*)rows, slot, (const __nv_bfloat16*)residual, (__nv_bfloat16*)out, T, k,
-      H, nullptr, 0, 0, nullptr, 0, nullptr);
-  return check_launch("unpermute_reduce");
+  return fm_unpermute_reduce_gated(rows, slot, residual, out, T, k, H, nullptr, 0, 0, nullptr, 0, nullptr, s);
 }
 
 extern "C" int fm_unpermute_reduce_gated(const void* rows, const int* slot, const void* residual,
@@ -717,13 +769,21 @@ extern "C" int fm_unpermute_reduce_gated(const void* rows, const int* slot, cons
                                          int wait_expected, unsigned long long* wait_ns,
                                          unsigned long long timeout_ns, int* status, cudaStream_t s) {
   if (H % 8 != 0 || k > 16 || wait_n > 256) {
-    fm_set_error("unpermute_reduce_gated: H must be a multiple of 8, k at most 16, at most 256 sources");
+    fm_set_error("unpermute_reduce: H must be a multiple of 8, k at most 16, at most 256 sources");
     return -1;
   }
-  fm::unpermute_reduce_kernel<<<grid_for(T, 8), 256, 0, s>>>(
-      (const __nv_bfloat16*)rows, slot, (const __nv_bfloat16*)residual, (__nv_bfloat16*)out, T, k,
-      H, wait_flags, wait_n, wait_expected, wait_ns, timeout_ns ? timeout_ns : 4000000000ull, status);
-  return check_launch("unpermute_reduce_gated");
+  auto launch = [&](auto kernel) {
+    kernel<<<grid_for((long long)T * (H / 8), 256), 256, 0, s>>>(
+        (const __nv_bfloat16*)rows, slot, (const __nv_bfloat16*)residual, (__nv_bfloat16*)out, T, k, H, wait_flags,
+        wait_n, wait_expected, wait_ns, timeout_ns ? timeout_ns : 4000000000ull, status);
+  };
+  if (k <= 1) launch(fm::unpermute_reduce_kernel<1>);
+  else if (k <= 2) launch(fm::unpermute_reduce_kernel<2>);
+  else if (k <= 4) launch(fm::unpermute_reduce_kernel<4>);
+  else if (k <= 6) launch(fm::unpermute_reduce_kernel<6>);
+  else if (k <= 8) launch(fm::unpermute_reduce_kernel<8>);
+  else launch(fm::unpermute_reduce_kernel<16>);
+  return check_launch("unpermute_reduce");
 }
 
 extern "C" int fm_adam(void* p, float* master, float* g, void* m, void* v, long long n, float lr,
