@@ -70,6 +70,25 @@ int fm_flash_attn_bwd_gated(const void* qkv, const void* out, const void* dout, 
 int fm_cross_entropy(void* logits, const long long* labels, float* loss_out, int T, int V,
                      float grad_scale, cudaStream_t s);
 
+// Router weight gradient dw [H, E] fp32 = x[T, H]^T (bf16) * dlogits[T, E] (fp32).  `partial` holds
+// fm_router_wgrad_splits(T, H, E) x H x E floats.
+int fm_router_wgrad_splits(int T, int H, int E);
+int fm_router_wgrad(const void* x, const float* dlogits, float* partial, float* dw, int T, int H, int E,
+                    cudaStream_t s);
+// main[ids[t]] += dy[t] (fp32 rows of H values, bf16 gradients; ids must be rows of `main`).
+int fm_embedding_grad(const long long* ids, const void* dy, float* main_grad, int T, int H, cudaStream_t s);
+// One Adam(W) launch over `count` tensors (see fm_adam for the update; no master copies).
+typedef struct {
+  void* p;
+  const float* g;
+  void* m;
+  void* v;
+  long long n;
+} FmAdamTensor;
+#define FM_ADAM_MAX_TENSORS 64
+int fm_adam_multi(const FmAdamTensor* tensors, int count, float lr, float beta1, float beta2, float eps,
+                  float weight_decay, int step, float grad_scale, int state_bf16, cudaStream_t s);
+
 // Padded-capacity routing plan (see moe_plan_kernel).  Outputs: sorted_indices [E*cap] int64,
 // slot_probs [E*cap] fp32, slot_of_token [T,k] int32, routed_per_expert [E] int32,
 // tokens_per_expert [E] int32 (== cap; may be null).

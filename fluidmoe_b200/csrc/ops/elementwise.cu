@@ -403,6 +403,26 @@ unpermute_reduce_kernel(const __nv_bfloat16* __restrict__ rows, const int* __res
 }
 
 // --------------------------------------------------------------------------------------------
+// Embedding gradient: main[ids[t]] += dy[t], one 16-byte piece of a bf16 row per thread, added to the fp32
+// row with two four-wide reductions.  Converting to fp32 first and adding element by element took 163 us
+// for 4096 tokens of 4096 columns, this takes 29.
+// --------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256)
+embedding_grad_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ dy,
+                      float* __restrict__ main_grad, long long total, int nvec) {
+  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
+       idx += (long long)gridDim.x * blockDim.x) {
+    const long long t = idx / nvec;
+    const int i = (int)(idx - t * nvec);
+    float v[8];
+    unpack8(reinterpret_cast<const uint4*>(dy)[idx], v);
+    float* dst = main_grad + (ids[t] * nvec + i) * 8;
+    red_add_v4_f32(dst, v[0], v[1], v[2], v[3]);
+    red_add_v4_f32(dst + 4, v[4], v[5], v[6], v[7]);
+  }
+}
+
+// --------------------------------------------------------------------------------------------
 // Fused Adam(W) on a flat slice: fp32 gradient, fp32 moments, bf16 parameter updated in place
 // (optionally through an fp32 master copy).  The gradient may be zeroed in the same pass.
 // --------------------------------------------------------------------------------------------
@@ -466,6 +486,68 @@ adam_kernel(__nv_bfloat16* __restrict__ p, float* __restrict__ master, float* __
     if (master) Vec4<float>::store(master + q, w);
     Vec4<__nv_bfloat16>::store(p + q, w);
     if (zero_grad) *reinterpret_cast<float4*>(g + q) = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+
+// The same update for many tensors in one launch: a model has some dozen small parameters, whose launches
+// cost more than their work.  The tensors lie side by side in chunks of kAdamChunk elements; a CTA finds its
+// chunk's tensor in the table of first chunks.  Tensors that are not aligned, and the last elements of each,
+// go element by element.
+constexpr int kAdamChunk = 512 * 4 * 4;
+struct AdamTable {
+  FmAdamTensor t[FM_ADAM_MAX_TENSORS];
+  int first[FM_ADAM_MAX_TENSORS + 1];
+  int count;
+};
+template <class ST>
+__global__ void __launch_bounds__(512)
+adam_multi_kernel(const __grid_constant__ AdamTable tab, float lr, float beta1, float beta2, float eps,
+                  float weight_decay, float rbc1, float rbc2, float grad_scale) {
+  for (int chunk = blockIdx.x; chunk < tab.first[tab.count]; chunk += gridDim.x) {
+    int lo = 0, hi = tab.count - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (tab.first[mid] <= chunk) lo = mid;
+      else hi = mid - 1;
+    }
+    const FmAdamTensor& t = tab.t[lo];
+    __nv_bfloat16* const p = reinterpret_cast<__nv_bfloat16*>(t.p);
+    const float* const g = t.g;
+    ST* const m = reinterpret_cast<ST*>(t.m);
+    ST* const v = reinterpret_cast<ST*>(t.v);
+    const long long begin = (long long)(chunk - tab.first[lo]) * kAdamChunk;
+    const long long end = min(t.n, begin + kAdamChunk);
+    const bool aligned = ((reinterpret_cast<uintptr_t>(p) & 7) | (reinterpret_cast<uintptr_t>(g) & 15) |
+                          (reinterpret_cast<uintptr_t>(m) & 15) | (reinterpret_cast<uintptr_t>(v) & 15)) == 0;
+    auto update = [&](float gj, float& w, float& mm, float& vv) {
+      gj *= grad_scale;
+      mm = beta1 * mm + (1.f - beta1) * gj;
+      vv = beta2 * vv + (1.f - beta2) * gj * gj;
+      w -= lr * ((mm * rbc1) / (sqrtf(vv * rbc2) + eps) + weight_decay * w);
+    };
+    if (aligned) {
+#pragma unroll 2
+      for (long long q = begin + threadIdx.x * 4; q + 4 <= end; q += 512 * 4) {
+        float gr[4], w[4], mm[4], vv[4];
+        Vec4<float>::load(g + q, gr);
+        Vec4<ST>::load(m + q, mm);
+        Vec4<ST>::load(v + q, vv);
+        Vec4<__nv_bfloat16>::load(p + q, w);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) update(gr[j], w[j], mm[j], vv[j]);
+        Vec4<ST>::store(m + q, mm);
+        Vec4<ST>::store(v + q, vv);
+        Vec4<__nv_bfloat16>::store(p + q, w);
+      }
+    }
+    // begin is a multiple of 4: what is left of an aligned tensor are at most three elements
+    for (long long q = (aligned ? begin + ((end - begin) & ~3ll) : begin) + threadIdx.x; q < end; q += 512) {
+      float w = __bfloat162float(p[q]), mm = (float)m[q], vv = (float)v[q];
+      update(g[q], w, mm, vv);
+      m[q] = (ST)mm;
+      v[q] = (ST)vv;
+      p[q] = __float2bfloat16(w);
+    }
   }
 }
 
@@ -824,6 +906,52 @@ extern "C" int fm_adam(void* p, float* master, float* g, void* m, void* v, long 
     return check_launch("adam_tail");
   }
   return 0;
+}
+
+extern "C" int fm_adam_multi(const FmAdamTensor* tensors, int count, float lr, float beta1, float beta2, float eps,
+                             float weight_decay, int step, float grad_scale, int state_bf16, cudaStream_t s) {
+  if (count < 0 || count > FM_ADAM_MAX_TENSORS) {
+    fm_set_error("adam_multi: too many tensors for one launch");
+    return -1;
+  }
+  fm::AdamTable tab;
+  tab.count = 0;
+  long long chunks = 0;
+  for (int i = 0; i < count; ++i) {
+    if (tensors[i].n <= 0) continue;
+    tab.t[tab.count] = tensors[i];
+    tab.first[tab.count++] = (int)chunks;
+    chunks += (tensors[i].n + fm::kAdamChunk - 1) / fm::kAdamChunk;
+    if (chunks > 2147483647ll - 148 * 8) {
+      fm_set_error("adam_multi: too many elements for one launch");
+      return -1;
+    }
+  }
+  if (tab.count == 0) return 0;
+  tab.first[tab.count] = (int)chunks;
+  const float rbc1 = 1.f / (1.f - powf(beta1, (float)step));
+  const float rbc2 = 1.f / (1.f - powf(beta2, (float)step));
+  const int grid = grid_for(chunks, 1, 148 * 4);
+  if (state_bf16)
+    fm::adam_multi_kernel<__nv_bfloat16><<<grid, 512, 0, s>>>(tab, lr, beta1, beta2, eps, weight_decay, rbc1, rbc2,
+                                                             grad_scale);
+  else
+    fm::adam_multi_kernel<float><<<grid, 512, 0, s>>>(tab, lr, beta1, beta2, eps, weight_decay, rbc1, rbc2,
+                                                     grad_scale);
+  return check_launch("adam_multi");
+}
+
+extern "C" int fm_embedding_grad(const long long* ids, const void* dy, float* main_grad, int T, int H,
+                                 cudaStream_t s) {
+  if (H % 8 != 0 || (reinterpret_cast<uintptr_t>(dy) & 15) || (reinterpret_cast<uintptr_t>(main_grad) & 15)) {
+    fm_set_error("embedding_grad: H must be a multiple of 8 and rows 16-byte aligned");
+    return -1;
+  }
+  const long long total = (long long)T * (H / 8);
+  if (total == 0) return 0;
+  fm::embedding_grad_kernel<<<grid_for(total, 256), 256, 0, s>>>(ids, (const __nv_bfloat16*)dy, main_grad, total,
+                                                                H / 8);
+  return check_launch("embedding_grad");
 }
 
 extern "C" int fm_router_bwd(const float* dprobs_slots, const int* slot_of_token, const long long* top_idx,

@@ -1,6 +1,7 @@
 // Router kernels: top-k + softmax, the padded-capacity plan and the dropless plan.  All three turn
 // [T, E] logits or [T, k] choices into a few small arrays; they sit between two GEMMs of every MoE
 // layer with nothing to overlap, so what counts is their latency, not their bandwidth.
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -570,6 +571,93 @@ dropless_place_kernel(const long long* __restrict__ top_idx, const float* __rest
   }
 }
 
+// --------------------------------------------------------------------------------------------
+// Router weight gradient dW[h, e] = sum_t x[t, h] * dlogits[t, e], x in bf16, everything else fp32 (the
+// gradient of the logits stays in 32 bits, so this is no job for the bf16 tensor cores).  A CTA owns 1024
+// columns of x (a thread four neighbours), EB experts and a share of the tokens; the gradients of the
+// logits are the same for all threads and come from shared memory four at a time.  The shares are summed in
+// a fixed order by a second kernel.  Against a conversion of x
+// to fp32 and a library product: 4096 x 4096, 8 experts, 109 -> 26 us; 8192 x 2048, 64 experts, 127 -> 83 us (the
+// fp32 pipe alone needs 31), with a third of the error.
+// --------------------------------------------------------------------------------------------
+constexpr int kRouterThreads = 256, kRouterTokens = 32;
+
+template <int EB>
+__global__ void __launch_bounds__(kRouterThreads, 2)
+router_wgrad_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ dl, float* __restrict__ partial,
+                    int T, int H, int E, int per_split) {
+  constexpr int kAhead = 8;      // rows of x in flight
+  __shared__ __align__(16) float dl_s[kRouterTokens][EB];
+  const int h = blockIdx.x * 4 * kRouterThreads + 4 * threadIdx.x;
+  const int e0 = blockIdx.y * EB;
+  const int t_end = min(T, (int)(blockIdx.z + 1) * per_split);
+  float acc[4][EB];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+#pragma unroll
+    for (int e = 0; e < EB; ++e) acc[q][e] = 0.f;
+  for (int t0 = blockIdx.z * per_split; t0 < t_end; t0 += kRouterTokens) {
+    const int nt = min(kRouterTokens, t_end - t0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < kRouterTokens * EB; i += kRouterThreads) {
+      const int t = i / EB, e = e0 + i % EB;
+      dl_s[t][i % EB] = (t < nt && e < E) ? dl[(long long)(t0 + t) * E + e] : 0.f;
+    }
+    __syncthreads();
+    if (h < H) {
+      const __nv_bfloat16* xr = x + (long long)t0 * H + h;
+      for (int t = 0; t < nt; t += kAhead) {
+        uint2 w[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+          w[u] = t + u < nt ? *reinterpret_cast<const uint2*>(xr + (long long)(t + u) * H) : make_uint2(0, 0);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          if (t + u >= nt) break;
+          const float xv[4] = {__uint_as_float(w[u].x << 16), __uint_as_float(w[u].x & 0xffff0000u),
+                               __uint_as_float(w[u].y << 16), __uint_as_float(w[u].y & 0xffff0000u)};
+#pragma unroll
+          for (int e = 0; e < EB; e += 4) {
+            const float4 d = *reinterpret_cast<const float4*>(&dl_s[t + u][e]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              acc[q][e] = fmaf(xv[q], d.x, acc[q][e]);
+              acc[q][e + 1] = fmaf(xv[q], d.y, acc[q][e + 1]);
+              acc[q][e + 2] = fmaf(xv[q], d.z, acc[q][e + 2]);
+              acc[q][e + 3] = fmaf(xv[q], d.w, acc[q][e + 3]);
+            }
+          }
+        }
+      }
+    }
+  }
+  if (h >= H) return;
+  float* out = partial + ((long long)blockIdx.z * H + h) * E + e0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+#pragma unroll
+    for (int e = 0; e < EB; e += 4) {
+      if (e0 + e + 4 <= E && E % 4 == 0) {
+        *reinterpret_cast<float4*>(out + (long long)q * E + e) =
+            make_float4(acc[q][e], acc[q][e + 1], acc[q][e + 2], acc[q][e + 3]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (e0 + e + i < E) out[(long long)q * E + e + i] = acc[q][e + i];
+      }
+    }
+}
+
+__global__ void __launch_bounds__(256)
+router_wgrad_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int splits, long long n) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float s = 0.f;
+#pragma unroll 8
+  for (int q = 0; q < splits; ++q) s += partial[q * n + i];
+  dw[i] = s;
+}
+
 }  // namespace fm
 
 static int check_launch(const char* what) {
@@ -581,6 +669,38 @@ static int check_launch(const char* what) {
     return (int)e;
   }
   return 0;
+}
+
+static int router_eb(int E) { return E <= 8 ? 8 : 16; }
+
+extern "C" int fm_router_wgrad_splits(int T, int H, int E) {
+  const int eb = router_eb(E);
+  const int tiles = ((H + 4 * fm::kRouterThreads - 1) / (4 * fm::kRouterThreads)) * ((E + eb - 1) / eb);
+  int splits = (2 * 148) / tiles;                                         // two CTAs an SM
+  const int most = (T + fm::kRouterTokens - 1) / fm::kRouterTokens;       // and a step's tokens for each
+  if (splits > most) splits = most;
+  return splits < 1 ? 1 : splits;
+}
+
+extern "C" int fm_router_wgrad(const void* x, const float* dlogits, float* partial, float* dw, int T, int H, int E,
+                               cudaStream_t s) {
+  if (T < 1 || E < 1 || H < 4 || H % 4 != 0 || (reinterpret_cast<uintptr_t>(x) & 7)) {
+    fm_set_error("router_wgrad: a multiple of four columns, 8-byte aligned");
+    return -1;
+  }
+  const int splits = fm_router_wgrad_splits(T, H, E), eb = router_eb(E);
+  const int per = (T + splits - 1) / splits;
+  const dim3 grid((H + 4 * fm::kRouterThreads - 1) / (4 * fm::kRouterThreads), (E + eb - 1) / eb, splits);
+  auto launch = [&](auto kernel) {
+    kernel<<<grid, fm::kRouterThreads, 0, s>>>((const __nv_bfloat16*)x, dlogits, partial, T, H, E, per);
+  };
+  if (eb == 8) launch(fm::router_wgrad_kernel<8>);
+  else launch(fm::router_wgrad_kernel<16>);
+  int rc = check_launch("router_wgrad");
+  if (rc) return rc;
+  const long long n = (long long)H * E;
+  fm::router_wgrad_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(partial, dw, splits, n);
+  return check_launch("router_wgrad_reduce");
 }
 
 extern "C" int fm_topk_softmax(const float* logits, long long* idx, float* probs, int T, int E,

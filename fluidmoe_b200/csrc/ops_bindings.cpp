@@ -1,8 +1,11 @@
 // pybind11 bindings of the element-wise kernels.
 #include <pybind11/pybind11.h>
+#include <pybind11/stl.h>
 
 #include <stdexcept>
 #include <string>
+#include <tuple>
+#include <vector>
 
 #include "include/fm_api.h"
 #include "include/fm_ops.h"
@@ -65,6 +68,28 @@ void bind_ops(py::module_& m) {
     chk(fm_moe_plan(p<const long long*>(ti), p<const float*>(tp), T, k, E, cap, p<long long*>(si),
                     p<float*>(sp), p<int*>(sot), p<int*>(rpe), p<int*>(tpe), st(s)), "moe_plan");
   });
+  m.def("router_wgrad_splits", &fm_router_wgrad_splits);
+  m.def("router_wgrad", [](u x, u dl, u partial, u dw, int T, int H, int E, u s) {
+    chk(fm_router_wgrad(p<const void*>(x), p<const float*>(dl), p<float*>(partial), p<float*>(dw), T, H, E, st(s)),
+        "router_wgrad");
+  });
+  m.def("embedding_grad", [](u ids, u dy, u main_grad, int T, int H, u s) {
+    chk(fm_embedding_grad(p<const long long*>(ids), p<const void*>(dy), p<float*>(main_grad), T, H, st(s)),
+        "embedding_grad");
+  });
+  // tensors: (parameter, gradient, first moment, second moment, elements) per entry
+  m.def("adam_multi", [](const std::vector<std::tuple<u, u, u, u, long long>>& tensors, float lr, float b1, float b2,
+                         float eps, float wd, int step, float gs, int state_bf16, u s) {
+    FmAdamTensor tab[FM_ADAM_MAX_TENSORS];
+    for (size_t i = 0; i < tensors.size();) {
+      int n = 0;
+      for (; n < FM_ADAM_MAX_TENSORS && i < tensors.size(); ++n, ++i)
+        tab[n] = {p<void*>(std::get<0>(tensors[i])), p<const float*>(std::get<1>(tensors[i])),
+                  p<void*>(std::get<2>(tensors[i])), p<void*>(std::get<3>(tensors[i])), std::get<4>(tensors[i])};
+      chk(fm_adam_multi(tab, n, lr, b1, b2, eps, wd, step, gs, state_bf16, st(s)), "adam_multi");
+    }
+  });
+  m.attr("ADAM_MAX_TENSORS") = FM_ADAM_MAX_TENSORS;
   m.def("dropless_plan_local", [](u ti, u tp, int T, int k, int E, int rows_max, u counts, u rows, u offs, u tok,
                                   u prob, u sot, u s) {
     chk(fm_dropless_plan_local(p<const long long*>(ti), p<const float*>(tp), T, k, E, rows_max, p<int*>(counts),

@@ -66,6 +66,10 @@ class _Embedding(torch.autograd.Function):
         flat_ids, flat_dy = ids.reshape(-1), dy.reshape(-1, dy.shape[-1])
         main = getattr(w, "main_grad", None)
         if main is not None and main.dtype == torch.float32:
+            if main.is_cuda and _native.available():
+                from ..ops import elementwise
+                if elementwise.embedding_grad_(main, flat_ids, flat_dy):
+                    return None, None
             main.index_add_(0, flat_ids, flat_dy.float())
             return None, None
         grad = torch.zeros_like(w, dtype=torch.float32).index_add_(0, flat_ids, flat_dy.float())

@@ -271,7 +271,7 @@ class TransformerLayerFunction(torch.autograd.Function):
                 d_ln2_router = (dlogits.to(router_w.dtype) @ router_w.detach().t()).to(dy2.dtype)
                 ln2_for_dw = ln2_out
                 sched.register_dw_task(f"layer{lid}.router", lid,
-                                       lambda: (ln2_for_dw.float().t() @ dlogits).to(torch.float32), router_w)
+                                       lambda: router_ops.router_wgrad(ln2_for_dw, dlogits), router_w)
                 d_ln2 = dl.unpermute(db, rplan, dperm, d_ln2_router, "dperm", waited=True)
             if w1_late:
                 moe_dropless.register_dw_tasks(rplan, st, dfc2_em, dpre_em, w1, w2, lid, f"layer{lid}.moe", which="w1")
@@ -293,7 +293,7 @@ class TransformerLayerFunction(torch.autograd.Function):
             d_ln2_router = (dlogits.to(router_w.dtype) @ router_w.detach().t()).to(dy2.dtype)
             ln2_for_dw = ln2_out
             sched.register_dw_task(f"layer{lid}.router", lid,
-                                   lambda: (ln2_for_dw.float().t() @ dlogits).to(torch.float32), router_w)
+                                   lambda: router_ops.router_wgrad(ln2_for_dw, dlogits), router_w)
             d_ln2 = permute.unpermute_reduce(dperm, rplan.slot_of_token, d_ln2_router)
         else:
             # ---- R1: combine gradient -> FC2 dX + activation backward ----
@@ -328,7 +328,7 @@ class TransformerLayerFunction(torch.autograd.Function):
                 ln2_for_dw = ln2_out
 
                 def router_dw():
-                    return (ln2_for_dw.float().t() @ dlogits).to(torch.float32)
+                    return router_ops.router_wgrad(ln2_for_dw, dlogits)
                 sched.register_dw_task(f"layer{lid}.router", lid, router_dw, router_w)
                 return d_router
 

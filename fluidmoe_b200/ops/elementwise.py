@@ -201,6 +201,52 @@ def dropless_plan_local(top_idx, top_probs, num_experts):
     return row_token, row_prob, slot_of_token, counts, group_rows, group_offs
 
 
+def router_wgrad(x, dlogits):
+    """``x[T, H]^T (bf16) @ dlogits[T, E] (fp32)`` -> [H, E] fp32; None when the kernel does not take these."""
+    if x.dtype != torch.bfloat16 or dlogits.dtype != torch.float32 or x.shape[1] % 4 or not x.is_contiguous() \
+            or x.shape[0] == 0 or x.data_ptr() % 8 or not dlogits.is_cuda:
+        return None
+    global LAUNCHES
+    T, H = x.shape
+    E = dlogits.shape[1]
+    dlogits = dlogits.contiguous()
+    lib = _native.lib()
+    partial = torch.empty(lib.router_wgrad_splits(T, H, E), H, E, dtype=torch.float32, device=x.device)
+    dw = torch.empty(H, E, dtype=torch.float32, device=x.device)
+    LAUNCHES += 1
+    lib.router_wgrad(x.data_ptr(), dlogits.data_ptr(), partial.data_ptr(), dw.data_ptr(), T, H, E, _s())
+    return dw
+
+
+def embedding_grad_(main, ids, dy) -> bool:
+    """``main[ids[t]] += dy[t]`` in place (fp32 rows, bf16 gradients); False when the kernel does not take these."""
+    if not (main.is_cuda and dy.is_cuda and ids.is_cuda) or main.dtype != torch.float32 or dy.dtype != torch.bfloat16 \
+            or ids.dtype != torch.int64 or main.shape[1] % 8 or not main.is_contiguous() or main.data_ptr() % 16:
+        return False
+    dy, ids = dy.contiguous(), ids.contiguous()
+    if dy.data_ptr() % 16:
+        return False
+    _native.lib().embedding_grad(ids.data_ptr(), dy.data_ptr(), main.data_ptr(), dy.shape[0], dy.shape[1], _s())
+    return True
+
+
+def adam_multi(tensors, state_bf16, lr, beta1, beta2, eps, weight_decay, step, grad_scale=1.0):
+    """Adam(W) over ``(p, g, m, v)`` tuples (bf16 parameters, fp32 gradients, moments of one type) with as
+    few launches as the kernel's table allows."""
+    global LAUNCHES
+    if not tensors:
+        return
+    entries = []
+    for p, g, m, v in tensors:
+        assert p.dtype == torch.bfloat16 and g.dtype == torch.float32 and m.dtype == v.dtype
+        _same_cuda_device(p, g, m, v)
+        entries.append((p.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr(), p.numel()))
+    lib = _native.lib()
+    LAUNCHES += (len(entries) - 1) // lib.ADAM_MAX_TENSORS
+    lib.adam_multi(entries, float(lr), float(beta1), float(beta2), float(eps), float(weight_decay), int(step),
+                   float(grad_scale), int(state_bf16), _s())
+
+
 def cross_entropy_(logits, labels, grad_scale):
     """In place: returns per-row losses (fp32) and leaves ``(softmax - onehot) * grad_scale`` in
     ``logits`` (bf16 [T, V], V a multiple of 8)."""

@@ -126,6 +126,16 @@ def build_dropless_plan(top_idx: torch.Tensor, top_probs: torch.Tensor, num_expe
                        slot_te.gather(1, top_idx).to(torch.int32), counts, counts, rmap, cap)
 
 
+def router_wgrad(x: torch.Tensor, dlogits: torch.Tensor) -> torch.Tensor:
+    """Router weight gradient ``x[T, H]^T @ dlogits[T, E]`` in fp32."""
+    if _native.use_native(x, dlogits):
+        from . import elementwise
+        res = elementwise.router_wgrad(x, dlogits)
+        if res is not None:
+            return res
+    return (x.float().t() @ dlogits).to(torch.float32)
+
+
 def router_backward_logits(dprobs_slots: torch.Tensor, plan: RoutingPlan, top_idx: torch.Tensor,
                            top_probs: torch.Tensor, logits: torch.Tensor, num_experts: int,
                            aux_loss_coeff: float = 0.0, z_loss_coeff: float = 0.0,

@@ -49,3 +49,53 @@ def test_unpermute(k, T, H, with_res):
         s = slot[:, j].long()
         acc = torch.where((s >= 0)[:, None], acc + rows[s.clamp(min=0)].float(), acc)
     assert torch.equal(got, acc.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("T", [1, 31, 33, 1531])
+@pytest.mark.parametrize("H,E", [(4, 1), (2, 3), (264, 8), (512, 16), (520, 17), (1028, 64), (2048, 70)])
+def test_router_weight_gradient(T, H, E):
+    from fluidmoe_b200.ops import router
+    torch.manual_seed(T + E)
+    x, dl = _rand(T, H), torch.randn(T, E, device="cuda")
+    got = router.router_wgrad(x, dl)
+    ref = x.double().t() @ dl.double()
+    # fp32 sums of T products in an order of their own
+    assert ((got.double() - ref).abs() <= 1e-6 * (x.double().abs().t() @ dl.double().abs()) + 1e-30).all()
+
+
+@pytest.mark.parametrize("T,V,H", [(1, 3, 8), (700, 5, 264), (513, 1000, 1024)])
+def test_embedding_gradient(T, V, H):
+    from fluidmoe_b200.ops import elementwise
+    torch.manual_seed(T)
+    ids, dy = torch.randint(0, V, (T,), device="cuda"), _rand(T, H)
+    main = torch.randn(V, H, device="cuda")
+    ref = main.double().index_add_(0, ids, dy.double())
+    terms = main.double().abs().index_add_(0, ids, dy.double().abs())
+    assert elementwise.embedding_grad_(main, ids, dy)
+    assert ((main.double() - ref).abs() <= 2e-6 * terms).all()
+
+
+@pytest.mark.parametrize("state", [torch.float32, torch.bfloat16])
+def test_adam_over_many_tensors_equals_one_by_one(state):
+    """More tensors than one launch's table holds, sizes around the chunk and off the vector width, one base
+    off its alignment.  The compiler may contract either kernel's products and sums into fused ones, which
+    saves a rounding of 2^-24 of a term; the terms of a moment have one sign or stay below 4 here."""
+    from fluidmoe_b200.ops import elementwise
+    torch.manual_seed(0)
+    sizes = [1, 3, 4, 5, 8191, 8192, 8193, 8195, 40000, 2] + [16] * 60
+    kw = dict(lr=1e-2, beta1=0.9, beta2=0.99, eps=1e-8, weight_decay=0.1, step=3, grad_scale=0.5)
+    sets = []
+    for off, n in enumerate(sizes):
+        lead = 1 if off == 6 else 0
+        mk = lambda t: torch.cat([torch.zeros(lead, device="cuda"), t]).to(state)[lead:]    # noqa: E731
+        p = torch.cat([torch.zeros(lead, device="cuda"), torch.randn(n, device="cuda")]).bfloat16()[lead:]
+        sets.append((p, torch.randn(n, device="cuda"), mk(torch.randn(n, device="cuda")), mk(torch.rand(n, device="cuda"))))
+    ones = [tuple(t.clone() if i != 6 else torch.cat([t[:1], t])[1:] for t in s) for i, s in enumerate(sets)]
+    for p, g, m, v in ones:
+        elementwise.adam_step(p, None, g, m, v, **kw)
+    elementwise.adam_multi(sets, state == torch.bfloat16, **kw)
+    for a, b in zip(sets, ones):
+        for x, y in zip(a, b):
+            # 4 * 2^-23 of absolute error in fp32 (four roundings), then one rounding of bf16
+            rtol = 0.0 if x.dtype == torch.float32 else 2.0 ** -7
+            torch.testing.assert_close(x.float(), y.float(), rtol=rtol, atol=4 * 2.0 ** -23 * 4)
