@@ -62,6 +62,9 @@ static void gemm_launch(const py::dict& d, uintptr_t stream) {
   g.out_fp32 = get<int>(d, "out_fp32", 0);
   g.accumulate = get<int>(d, "accumulate", 0);
   g.alpha = get<float>(d, "alpha", 1.0f);
+  g.alpha_dev = ptr<const float*>(d, "alpha_dev");
+  g.residual = ptr<const void*>(d, "residual");
+  g.ld_residual = get<long long>(d, "ld_residual", 0);
   g.act_out = ptr<void*>(d, "act_out");
   g.ld_act = get<long long>(d, "ld_act", 0);
   g.pre_out = ptr<void*>(d, "pre_out");

@@ -287,6 +287,9 @@ struct EpiStore {
   int accumulate;
   float alpha;
   int boxes;          // C can be written with bulk tensor stores: map 0 is C as [group][row][column]
+  const float* alpha_dev;
+  const __nv_bfloat16* residual;   // what a bf16 result is added to: another array, or C itself
+  long long ld_residual;
 
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
@@ -298,6 +301,7 @@ struct EpiStore {
     const long long goff = a.mode == 0 ? 0 : (long long)t.g * group_stride;
     const bool row_ok = r < t.rows_valid;
     const int rows_ok = max(0, min(32, t.rows_valid - (r - lane)));
+    const float alpha = alpha_dev != nullptr ? this->alpha * *alpha_dev : this->alpha;
     if (boxes) {
       // All 32 rows exist, or the boxes would reach into the next group's rows; columns past N are cut
       // off by the tensor map.
@@ -325,6 +329,27 @@ struct EpiStore {
           for (int c = chalf * kStep; c < (chalf + 1) * kStep; c += 2) {
             const int col = t.n_tile * BN + c * 32;
             if (col >= a.N) break;
+            if (residual != nullptr && col + 64 <= a.N) {
+              // The stage that turns the rows of the residual over to the lanes lies over the boxes.
+              uint32_t w[32];
+              if (lane == 0) bulk_wait_group_read<0>();
+              __syncwarp();
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                float v[32], p[32];
+                staged_load_bf16(stg, lane, p, 32, residual + row0 * ld_residual + col + 32 * h, ld_residual);
+                load_acc(taddr + (c + h) * 32, v, zero);
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                  w[16 * h + i] = pack_bf16x2(fmaf(v[2 * i], alpha, p[2 * i]), fmaf(v[2 * i + 1], alpha, p[2 * i + 1]));
+              }
+              __syncwarp();
+              uint8_t* box = bs.stg;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) bs.put(box, i, make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]));
+              bs.send(maps, box, col, (int)row0, z);
+              continue;
+            }
             uint8_t* box = bs.next<1>();
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -333,6 +358,16 @@ struct EpiStore {
               if (alpha != 1.0f) {
 #pragma unroll
                 for (int i = 0; i < 32; ++i) v[i] *= alpha;
+              }
+              if (residual != nullptr) {
+                // the last columns of the matrix
+                float p[32];
+                const int nc = min(32, a.N - col - 32 * h);
+                if (nc > 0) {
+                  load_row_bf16(residual + row * ld_residual + col + 32 * h, p, nc);
+#pragma unroll
+                  for (int i = 0; i < 32; ++i) v[i] += p[i];
+                }
               }
               bs.put_bf16(box, h, v);
             }
@@ -364,19 +399,22 @@ struct EpiStore {
         }
       } else {
         __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(C) + goff + row0 * ldc + col;
-        if (ncols == 32 && (ldc & 7) == 0 && aligned16(base)) {
-          if (accumulate) {
+        const __nv_bfloat16* src = accumulate ? base : residual ? residual + row0 * ld_residual + col : nullptr;
+        const long long ldr = accumulate ? ldc : ld_residual;
+        if (ncols == 32 && (ldc & 7) == 0 && aligned16(base) &&
+            (src == nullptr || ((ldr & 7) == 0 && aligned16(src)))) {
+          if (src != nullptr) {
             float p[32];
-            staged_load_bf16(stg, lane, p, rows_ok, base, ldc);
+            staged_load_bf16(stg, lane, p, rows_ok, src, ldr);
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] += p[i];
           }
           staged_store_bf16(stg, lane, v, rows_ok, base, ldc);
         } else if (row_ok) {
           __nv_bfloat16* dst = base + (long long)lane * ldc;
-          if (accumulate) {
+          if (src != nullptr) {
             float p[32];
-            load_row_bf16(dst, p, ncols);
+            load_row_bf16(src + (long long)lane * ldr, p, ncols);
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] += p[i];
           }
@@ -1547,9 +1585,21 @@ extern "C" int fm_gemm_launch(const FmGemmDesc* d, cudaStream_t stream) {
   switch (d->epi) {
     case FM_EPI_STORE: {
       EpiStore e{d->C, d->ldc, d->c_group_stride, d->out_fp32, d->accumulate,
-                 d->alpha == 0.f ? 1.0f : d->alpha, 0};
-      // The sums of an accumulating store are read first, so those keep the stores from registers.
-      if (!d->accumulate)
+                 d->alpha == 0.f ? 1.0f : d->alpha, 0, d->alpha_dev,
+                 reinterpret_cast<const __nv_bfloat16*>(d->residual), d->ld_residual};
+      if (d->residual != nullptr && (d->out_fp32 || d->accumulate || d->mode != 0)) {
+        set_err("a residual goes with a bf16 result that does not accumulate");
+        return -1;
+      }
+      if (d->accumulate && !d->out_fp32 && d->mode == 0) {
+        e.accumulate = 0;
+        e.residual = reinterpret_cast<const __nv_bfloat16*>(d->C);
+        e.ld_residual = d->ldc;
+      }
+      // Other sums that a store accumulates into are read first and keep the stores from registers; so does a
+      // residual off 16 bytes.
+      if (!e.accumulate &&
+          (e.residual == nullptr || (e.ld_residual % 8 == 0 && (reinterpret_cast<uintptr_t>(e.residual) & 15) == 0)))
         e.boxes = make_out_map(&maps.m[0], d->C, d->out_fp32 != 0, d->N,
                                d->mode == 0 ? (d->a_mn ? d->a_inner : d->a_outer) : d->M, d->ldc,
                                d->mode == 0 ? 1 : d->num_groups, d->c_group_stride);

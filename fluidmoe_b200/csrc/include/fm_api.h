@@ -48,6 +48,9 @@ typedef struct FmGemmDesc {
   int out_fp32;
   int accumulate;
   float alpha;
+  const float* alpha_dev;  // FM_EPI_STORE: device scalar that alpha is multiplied with (may be null)
+  const void* residual;    // FM_EPI_STORE, bf16 output, no accumulate: added before the one rounding (may be null)
+  long long ld_residual;
   // FM_EPI_ACT
   void* act_out;
   long long ld_act;

@@ -147,6 +147,8 @@ def output_projection_forward(attn_out: torch.Tensor, proj_weight: torch.Tensor,
     def with_residual(a_in, w):
         if residual is None:
             return project(a_in, w)
+        if residual.is_cuda and residual.dtype == torch.bfloat16 and residual.dim() == 2 and residual.stride(1) == 1:
+            return gemm.gemm_nt(a_in, w, residual=residual)
         out = residual.clone()
         return project(a_in, w, out=out, accumulate=True)
 
@@ -314,9 +316,9 @@ def hp2sp_qkv_backward(dqkv_hp: torch.Tensor, qkv_weight: torch.Tensor, plan: CP
 
 
 def _register_dense_dw(name: str, layer_id: int, x: torch.Tensor, dy: torch.Tensor, param,
-                       transpose_out: bool = False) -> None:
+                       transpose_out: bool = False, alpha_dev: Optional[torch.Tensor] = None) -> None:
     """Queue ``dW = dy^T @ x`` (``[N, K]``, the nn.Linear layout) or ``x^T @ dy`` when
-    ``transpose_out`` (``[K, N]``)."""
+    ``transpose_out`` (``[K, N]``), times the device scalar ``alpha_dev`` when there is one."""
     sched = get_backward_scheduler()
 
     def run():
@@ -326,9 +328,9 @@ def _register_dense_dw(name: str, layer_id: int, x: torch.Tensor, dy: torch.Tens
                 and a.dtype == torch.bfloat16 and bm.shape[1] % 8 == 0 and a.shape[1] % 8 == 0:
             first = not getattr(param, "_ar_buf_written", False)
             gemm.grouped_gemm_wgrad(a, bm, 1, out=param.main_grad, accumulate=not first,
-                                    max_ctas=sched.dw_max_ctas)
+                                    max_ctas=sched.dw_max_ctas, alpha_dev=alpha_dev)
             return None
-        return gemm.grouped_gemm_wgrad(a, bm, 1).view(param.shape)
+        return gemm.grouped_gemm_wgrad(a, bm, 1, alpha_dev=alpha_dev).view(param.shape)
 
     sched.register_dw_task(name, layer_id, run, param)
 

@@ -186,7 +186,10 @@ class TransformerLayerFunction(torch.autograd.Function):
             if shared_w1 is not None:
                 sh_act, sh_pre = gemm.grouped_gemm_act(ln2_out, shared_w1.unsqueeze(0), None,
                                                        activation=L.shared_activation, save_pre=needs_grad)
-                residual = gemm.gemm_nn(sh_act, shared_w2, out=h1.clone(), accumulate=True)
+                if h1.is_cuda and h1.dtype == torch.bfloat16:
+                    residual = gemm.gemm_nn(sh_act, shared_w2, residual=h1)
+                else:
+                    residual = gemm.gemm_nn(sh_act, shared_w2, out=h1.clone(), accumulate=True)
             with nvtx_range("unpermute"):
                 if mode_moe == "dropless_fused":
                     out = fused.dropless.unpermute(fused._buf(ep), rplan, combined, residual, "combined")

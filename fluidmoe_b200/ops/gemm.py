@@ -124,6 +124,8 @@ def grouped_gemm(
     gate: Optional[dict] = None,
     max_ctas: int = 0,
     zero_fill: bool = True,
+    residual: Optional[torch.Tensor] = None,
+    alpha_dev: Optional[torch.Tensor] = None,
 ) -> torch.Tensor:
     """``out[rows_g] = a[rows_g] @ B_g`` for every group g.
 
@@ -131,7 +133,9 @@ def grouped_gemm(
     group.  Rows of group g are ``[group_offs[g], group_offs[g] + group_rows[g])`` (device int32
     tensors, no host sync) or ``uniform_rows`` consecutive rows per group.  Rows outside every group
     are zero in a result allocated here, or undefined when the caller never reads them
-    (``zero_fill=False``, native kernel only).
+    (``zero_fill=False``, native kernel only).  ``residual`` (rows and type of a result without
+    ``accumulate``) is added before the result is rounded; ``alpha_dev``, an fp32 scalar on the device, is
+    multiplied with ``alpha``.
     """
     b3 = b if b.dim() == 3 else b.unsqueeze(0)
     G = b3.shape[0]
@@ -144,7 +148,15 @@ def grouped_gemm(
     if out is None:
         holes = group_rows is not None and (zero_fill or not _native.use_native(a, b))
         out = (torch.zeros if holes else torch.empty)(a.shape[0], N, dtype=out_dtype, device=a.device)
+    if residual is not None:
+        assert not accumulate and residual.shape == out.shape and residual.dtype == out.dtype == torch.bfloat16 \
+            and residual.stride(1) == 1 or not a.is_cuda
     if not _native.use_native(a, b):
+        if alpha_dev is not None:
+            alpha = alpha * float(alpha_dev)
+        if residual is not None:
+            out.copy_(residual)
+            accumulate = True
         for g, o, r in _groups(a.shape[0], G, group_rows, group_offs, uniform_rows, group_b):
             if r == 0:
                 continue
@@ -163,11 +175,20 @@ def grouped_gemm(
         out_fp32=int(out.dtype == torch.float32), accumulate=int(accumulate), alpha=float(alpha),
         max_ctas=max_ctas, status=status_buffer(a.device).data_ptr(),
     )
+    if residual is not None:
+        desc.update(residual=residual.data_ptr(), ld_residual=residual.stride(0))
+    if alpha_dev is not None:
+        desc["alpha_dev"] = _device_scalar(alpha_dev, a)
     desc.update(_group_kw(group_rows, group_offs, uniform_rows or 0, group_b))
     if gate:
         desc.update(gate)
     _launch(desc)
     return out
+
+
+def _device_scalar(t: torch.Tensor, like: torch.Tensor) -> int:
+    assert t.dtype == torch.float32 and t.numel() == 1 and t.device == like.device, (t.dtype, t.shape, t.device)
+    return t.data_ptr()
 
 
 def gemm_nt(a: torch.Tensor, w: torch.Tensor, **kw) -> torch.Tensor:
@@ -343,6 +364,7 @@ def grouped_gemm_wgrad(
     accumulate: bool = False,
     alpha: float = 1.0,
     max_ctas: int = 0,
+    alpha_dev: Optional[torch.Tensor] = None,
 ) -> torch.Tensor:
     """``out[g] (+)= a[rows_g]^T @ dy[rows_g]`` -> [G, M, N] (weight-gradient shape).
 
@@ -350,6 +372,7 @@ def grouped_gemm_wgrad(
     (the contraction runs in 64-row blocks); group offsets must be multiples of 64 or the
     groups must tile the buffer exactly.  fp32 ``out`` with ``accumulate=True`` adds straight
     into a gradient buffer (fluid/moe/backward.py:541-573, fluid/core/scheduler.py:188-213).
+    ``alpha_dev``: see ``grouped_gemm``.
     """
     rows, M = a.shape
     N = dy.shape[1]
@@ -362,6 +385,8 @@ def grouped_gemm_wgrad(
         accumulate = False
     o3 = out.view(G, M, N)
     if not _native.use_native(a, dy):
+        if alpha_dev is not None:
+            alpha = alpha * float(alpha_dev)
         for g, o, r in _groups(rows, G, group_rows, group_offs, uniform_rows):
             res = alpha * (a[o:o + r].float().t() @ dy[o:o + r].float())
             o3[g] = (o3[g].float() + res if accumulate else res).to(out.dtype)
@@ -377,6 +402,8 @@ def grouped_gemm_wgrad(
         out_fp32=int(out.dtype == torch.float32), accumulate=int(accumulate), alpha=float(alpha),
         max_ctas=max_ctas, status=status_buffer(a.device).data_ptr(),
     )
+    if alpha_dev is not None:
+        desc["alpha_dev"] = _device_scalar(alpha_dev, a)
     kw = _group_kw(group_rows, group_offs, uniform_rows or 0)
     kw.pop("num_groups", None)
     desc.update(kw)

@@ -394,3 +394,30 @@ def test_activation_epilogues_at_ragged_groups_and_edges(act, rows, F, cta_pair,
         (dz,) = torch.autograd.grad(y, z, d * p)
         close(dpre[r], dz)
         close(dprobs[r], (d * y.detach()).sum(1), rel=1e-5)
+
+
+@pytest.mark.parametrize("M,N,K", [(32, 128, 64), (31, 264, 64), (33, 40, 128), (257, 328, 64), (512, 192, 128)])
+@pytest.mark.parametrize("how", ["whole", "columns", "unaligned", "in place"])
+@pytest.mark.parametrize("cta_pair", [0, 1])
+def test_residual_and_device_scalar(M, N, K, how, cta_pair, monkeypatch):
+    """``alpha * alpha_dev * a @ w + residual`` with one rounding, for residuals of any row stride and base and
+    for the accumulating form, which reads C itself."""
+    monkeypatch.setattr(gemm, "CTA_PAIR", cta_pair)
+    torch.manual_seed(M + N)
+    a, w = _rand(M, K), _rand(N, K)
+    scale = torch.tensor(0.375, device="cuda")
+    lead = {"whole": 0, "columns": 8, "unaligned": 1, "in place": 0}[how]
+    r = _rand(M + 1, N + 16)[1:, lead:lead + N]
+    ref = 0.5 * 0.375 * (a.double() @ w.double().t()) + r.double()
+    if how == "in place":
+        out = gemm.grouped_gemm(a, w, b_layout="nk", out=r, accumulate=True, alpha=0.5, alpha_dev=scale)
+    else:
+        out = gemm.grouped_gemm(a, w, b_layout="nk", residual=r, alpha=0.5, alpha_dev=scale)
+    g = gemm.grouped_gemm_wgrad(a, _rand(M, 72).fill_(1.0), 1, alpha_dev=scale) if M % 64 == 0 else None
+    torch.cuda.synchronize()
+    gemm.check_status()
+    # fp32 sums of K products, then one rounding: 2^-8 of the value
+    assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * K ** 0.5).all()
+    if g is not None:
+        want = 0.375 * a.double().sum(0)[:, None].expand(K, 72)
+        assert ((g[0].double() - want).abs() <= 1e-5 * a.double().abs().sum(0)[:, None]).all()
