@@ -271,7 +271,7 @@ class TransformerLayerFunction(torch.autograd.Function):
                 dlogits = router_ops.router_backward_logits(
                     db.dprobs_perm.local, rplan, top_idx, top_probs, logits, L.num_experts, L.aux_loss_coeff,
                     L.z_loss_coeff, tpe_global, T * cp.cp_size)
-                d_ln2_router = (dlogits.to(router_w.dtype) @ router_w.detach().t()).to(dy2.dtype)
+                d_ln2_router = router_ops.router_dgrad(dlogits, router_w, dy2.dtype)
                 ln2_for_dw = ln2_out
                 sched.register_dw_task(f"layer{lid}.router", lid,
                                        lambda: router_ops.router_wgrad(ln2_for_dw, dlogits), router_w)
@@ -293,7 +293,7 @@ class TransformerLayerFunction(torch.autograd.Function):
             dlogits = router_ops.router_backward_logits(
                 dprobs_perm, rplan, top_idx, top_probs, logits, L.num_experts, L.aux_loss_coeff,
                 L.z_loss_coeff, tpe_global, T * cp.cp_size)
-            d_ln2_router = (dlogits.to(router_w.dtype) @ router_w.detach().t()).to(dy2.dtype)
+            d_ln2_router = router_ops.router_dgrad(dlogits, router_w, dy2.dtype)
             ln2_for_dw = ln2_out
             sched.register_dw_task(f"layer{lid}.router", lid,
                                    lambda: router_ops.router_wgrad(ln2_for_dw, dlogits), router_w)
@@ -327,7 +327,7 @@ class TransformerLayerFunction(torch.autograd.Function):
                 dlogits = router_ops.router_backward_logits(
                     dprobs_perm, rplan, top_idx, top_probs, logits, L.num_experts, L.aux_loss_coeff,
                     L.z_loss_coeff, tpe_global, T * cp.cp_size)
-                d_router = (dlogits.to(router_w.dtype) @ router_w.detach().t()).to(dy2.dtype)
+                d_router = router_ops.router_dgrad(dlogits, router_w, dy2.dtype)
                 ln2_for_dw = ln2_out
 
                 def router_dw():

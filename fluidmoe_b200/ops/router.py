@@ -126,6 +126,17 @@ def build_dropless_plan(top_idx: torch.Tensor, top_probs: torch.Tensor, num_expe
                        slot_te.gather(1, top_idx).to(torch.int32), counts, counts, rmap, cap)
 
 
+def router_dgrad(dlogits: torch.Tensor, router_weight: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """Gradient of the router input: ``dlogits[T, E] @ Wr[H, E]^T`` with operands in the weight's type."""
+    w = router_weight.detach()
+    d = dlogits.to(w.dtype)
+    if _native.use_native(d, w) and w.dtype == dtype == torch.bfloat16 and w.shape[1] % 8 == 0 and w.shape[0] % 8 == 0 \
+            and w.stride(1) == 1 and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0:
+        from .gemm import gemm_nt
+        return gemm_nt(d, w)
+    return (d @ w.t()).to(dtype)
+
+
 def router_wgrad(x: torch.Tensor, dlogits: torch.Tensor) -> torch.Tensor:
     """Router weight gradient ``x[T, H]^T @ dlogits[T, E]`` in fp32."""
     if _native.use_native(x, dlogits):

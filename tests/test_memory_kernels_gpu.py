@@ -99,3 +99,14 @@ def test_adam_over_many_tensors_equals_one_by_one(state):
             # 4 * 2^-23 of absolute error in fp32 (four roundings), then one rounding of bf16
             rtol = 0.0 if x.dtype == torch.float32 else 2.0 ** -7
             torch.testing.assert_close(x.float(), y.float(), rtol=rtol, atol=4 * 2.0 ** -23 * 4)
+
+
+@pytest.mark.parametrize("T,H,E", [(1, 8, 8), (33, 264, 16), (700, 2048, 64), (257, 512, 12)])
+def test_router_input_gradient(T, H, E):
+    from fluidmoe_b200.ops import router
+    torch.manual_seed(T)
+    dl, w = torch.randn(T, E, device="cuda"), _rand(H, E)
+    got = router.router_dgrad(dl, w, torch.bfloat16)
+    ref = dl.bfloat16().double() @ w.double().t()
+    # fp32 sums of E products, then one rounding of bf16
+    assert ((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * E ** 0.5).all()
