@@ -110,3 +110,22 @@ def test_router_input_gradient(T, H, E):
     ref = dl.bfloat16().double() @ w.double().t()
     # fp32 sums of E products, then one rounding of bf16
     assert ((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * E ** 0.5).all()
+
+
+@pytest.mark.parametrize("s,b,G,qpg,d,rot", [(1, 1, 1, 1, 128, 128), (37, 2, 3, 5, 64, 32), (65, 3, 2, 4, 128, 128), (300, 1, 1, 8, 128, 64)])
+@pytest.mark.parametrize("backward", [False, True])
+def test_rope(s, b, G, qpg, d, rot, backward):
+    """Angles of the two halves differ here, as the layout allows; the value head stays as it was."""
+    from fluidmoe_b200.ops import rope
+    torch.manual_seed(s)
+    x, f = _rand(s, b, G, (qpg + 2) * d), torch.randn(s, 1, 1, rot, device="cuda")
+    got = rope.rope_packed_(x.clone(), f, qpg, d, backward=backward).view(s, b, G, qpg + 2, d)
+    v = x.view(s, b, G, qpg + 2, d).double()
+    c, sn = torch.cos(f.double()).view(s, 1, 1, 1, rot), torch.sin(f.double()).view(s, 1, 1, 1, rot)
+    (c1, c2), (s1, s2) = c.chunk(2, -1), sn.chunk(2, -1)
+    x1, x2 = v[..., :rot].chunk(2, -1)
+    o = (x1 * c1 + x2 * s2, x2 * c2 - x1 * s1) if backward else (x1 * c1 - x2 * s1, x2 * c2 + x1 * s2)
+    ref = torch.cat((*o, v[..., rot:]), -1)
+    ref[..., -1, :] = v[..., -1, :]
+    assert ((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all()
+    assert torch.equal(got[..., -1, :], x.view(s, b, G, qpg + 2, d)[..., -1, :])
