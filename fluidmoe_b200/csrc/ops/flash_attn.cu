@@ -1270,24 +1270,43 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const _
   // first consumer of the output gradient that peers fill (SP -> HP exchange of the backward pass)
   if (wait_flags != nullptr)
     wait_counters_cta(wait_flags, wait_n, wait_expected, wait_ns, timeout_ns, status, kKernelIdDeltaWait);
-  // one warp per (row, batch, head): delta[b, h, row] = sum_d dO * O   (d == 128)
-  const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  // delta[b, h, row] = sum_d dO * O (d == 128): half a warp per (row, batch, head), eight of them per warp with
+  // all their loads in flight.  With one per warp and
+  // 8-byte loads the whole backward of 4096 positions, 32 heads took 510 us, now 498.
+  constexpr int kPairs = 4;
+  const int lane = threadIdx.x & 31, sub = lane & 15;
+  const long long w0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (2 * kPairs) + (lane >> 4);
   const long long total = (long long)s * b * hq;
-  if (w >= total) return;
-  const int lane = threadIdx.x & 31;
-  const uint2 o = reinterpret_cast<const uint2*>(out + w * kFaD)[lane];
-  const uint2 g = reinterpret_cast<const uint2*>(dout + w * kFaD)[lane];
-  const __nv_bfloat162 o0 = *reinterpret_cast<const __nv_bfloat162*>(&o.x);
-  const __nv_bfloat162 o1 = *reinterpret_cast<const __nv_bfloat162*>(&o.y);
-  const __nv_bfloat162 g0 = *reinterpret_cast<const __nv_bfloat162*>(&g.x);
-  const __nv_bfloat162 g1 = *reinterpret_cast<const __nv_bfloat162*>(&g.y);
-  float acc = __low2float(o0) * __low2float(g0) + __high2float(o0) * __high2float(g0) +
-              __low2float(o1) * __low2float(g1) + __high2float(o1) * __high2float(g1);
+  uint4 o[kPairs], g[kPairs];
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-  if (lane == 0) {
-    const long long h = w % hq, bb = (w / hq) % b, row = w / ((long long)hq * b);
-    delta[(bb * hq + h) * s + row] = acc;
+  for (int u = 0; u < kPairs; ++u) {
+    const long long w = w0 + 2 * u;
+    o[u] = g[u] = make_uint4(0, 0, 0, 0);
+    if (w < total) {
+      o[u] = reinterpret_cast<const uint4*>(out + w * kFaD)[sub];
+      g[u] = reinterpret_cast<const uint4*>(dout + w * kFaD)[sub];
+    }
+  }
+  float mine = 0.f;
+#pragma unroll
+  for (int u = 0; u < kPairs; ++u) {
+    const uint32_t ow[4] = {o[u].x, o[u].y, o[u].z, o[u].w}, gw[4] = {g[u].x, g[u].y, g[u].z, g[u].w};
+    float acc = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      acc = fmaf(__uint_as_float(ow[i] << 16), __uint_as_float(gw[i] << 16), acc);
+      acc = fmaf(__uint_as_float(ow[i] & 0xffff0000u), __uint_as_float(gw[i] & 0xffff0000u), acc);
+    }
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (sub == u) mine = acc;
+  }
+  const long long w = w0 + 2 * sub;
+  if (sub < kPairs && w < total) {
+    const long long rb = w / hq;
+    const int h = (int)(w - rb * hq);
+    const long long row = rb / b;
+    delta[((rb - row * b) * hq + h) * s + row] = mine;
   }
 }
 
@@ -2320,7 +2339,7 @@ extern "C" int fm_flash_attn_bwd_gated(const void* qkv, const void* out, const v
     return -3;
   }
   const long long nrows = (long long)s * b * hq;
-  fm::attn_delta_kernel<<<(unsigned)((nrows + 7) / 8), 256, 0, stream>>>(
+  fm::attn_delta_kernel<<<(unsigned)((nrows + 63) / 64), 256, 0, stream>>>(
       reinterpret_cast<const __nv_bfloat16*>(out), reinterpret_cast<const __nv_bfloat16*>(dout), delta, s, b, hq,
       wait_flags, wait_n, wait_expected, wait_ns, timeout_ns ? timeout_ns : 4000000000ull, status);
   constexpr int smem = 6 * fm::kTileBytes + 1024 + 256;

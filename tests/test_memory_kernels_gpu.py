@@ -129,3 +129,21 @@ def test_rope(s, b, G, qpg, d, rot, backward):
     ref[..., -1, :] = v[..., -1, :]
     assert ((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all()
     assert torch.equal(got[..., -1, :], x.view(s, b, G, qpg + 2, d)[..., -1, :])
+
+
+@pytest.mark.parametrize("T", [1, 295, 593, 1500])
+@pytest.mark.parametrize("H", [8, 520, 2048, 2056, 4104, 8192, 8200])
+@pytest.mark.parametrize("kind", ["rmsnorm", "layernorm", "layernorm without bias"])
+def test_norm_forward(T, H, kind):
+    torch.manual_seed(T + H)
+    x, w = _rand(T, H) + 0.5, _rand(H)
+    b = _rand(H) if kind == "layernorm" else None
+    y, mean, rstd = norm.norm_fwd(x, w, b, 1e-5, kind.split()[0])
+    xd = x.double()
+    mu = xd.mean(-1, keepdim=True) if kind != "rmsnorm" else torch.zeros(T, 1, device="cuda", dtype=torch.float64)
+    r = torch.rsqrt((xd - mu).pow(2).mean(-1, keepdim=True) + 1e-5)
+    ref = (xd - mu) * r * w.double() + (b.double() if b is not None else 0.0)
+    # fp32 sums of H terms, then one rounding of bf16
+    assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * ref.abs().max()).all()
+    assert ((rstd.double() - r.squeeze(1)).abs() <= 1e-5 * r.squeeze(1)).all()
+    assert mean is None or ((mean.double() - mu.squeeze(1)).abs() <= 1e-5).all()
