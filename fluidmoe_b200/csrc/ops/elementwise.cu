@@ -213,7 +213,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 // --------------------------------------------------------------------------------------------
 // Normalisation backward.  Each CTA walks rows blockIdx.x, +gridDim.x, ...; a thread owns the
 // same columns in every row, so the weight / bias gradients accumulate in registers and are
-// written once per CTA to a partial buffer [gridDim.x, 2, H] (RMSNorm: [gridDim.x, H]) that a second
+// written once per CTA to a partial buffer [gridDim.x, 2, H] (without a bias: [gridDim.x, H]) that a second
 // kernel reduces.  dx optionally adds the gradient that reaches the input through the residual branch.
 // Bound by memory (8 bytes an element with the residual): the loads of the next row are issued before the
 // one barrier of the current row, both sums cross it together, and what the second half needs is
@@ -225,7 +225,7 @@ constexpr int kNormBwdBlocks = 2 * 148;
 
 // kChunks (1, 2 or 4) is chosen from H: the per-thread arrays below are sized by it; one or two chunks fit
 // two CTAs per SM.
-template <int kChunks, bool kLayerNorm>
+template <int kChunks, bool kLayerNorm, bool kBias>
 __global__ void __launch_bounds__(kNormThreads, kChunks <= 2 ? 2 : 1)
 norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                 const __nv_bfloat16* __restrict__ w, const float* __restrict__ mean,
@@ -234,7 +234,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
   constexpr int kWarps = kNormThreads / 32;
   __shared__ float2 red[2][kWarps];
   const int nvec = H / 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float dg[kChunks][8], db[kLayerNorm ? kChunks : 1][8];
+  float dg[kChunks][8], db[kBias ? kChunks : 1][8];
   uint4 pw[kChunks];
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
@@ -243,7 +243,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       dg[c][j] = 0.f;
-      if (kLayerNorm) db[c][j] = 0.f;
+      if (kBias) db[c][j] = 0.f;
     }
   }
   uint4 px[kChunks], pd[kChunks], pr[kChunks];
@@ -286,7 +286,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
         s.y += gy;
         if (in) {
           dg[c][j] += dv[j] * xh;
-          if (kLayerNorm) db[c][j] += dv[j];
+          if (kBias) db[c][j] += dv[j];
         }
       }
     }
@@ -327,14 +327,14 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
       }
     }
   }
-  float* pg = partial + (long long)blockIdx.x * (kLayerNorm ? 2 : 1) * H;
+  float* pg = partial + (long long)blockIdx.x * (kBias ? 2 : 1) * H;
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
     const int i = threadIdx.x + c * kNormThreads;
     if (i < nvec) {
       *reinterpret_cast<float4*>(pg + i * 8) = make_float4(dg[c][0], dg[c][1], dg[c][2], dg[c][3]);
       *reinterpret_cast<float4*>(pg + i * 8 + 4) = make_float4(dg[c][4], dg[c][5], dg[c][6], dg[c][7]);
-      if (kLayerNorm) {
+      if (kBias) {
         *reinterpret_cast<float4*>(pg + H + i * 8) = make_float4(db[c][0], db[c][1], db[c][2], db[c][3]);
         *reinterpret_cast<float4*>(pg + H + i * 8 + 4) = make_float4(db[c][4], db[c][5], db[c][6], db[c][7]);
       }
@@ -904,17 +904,22 @@ extern "C" int fm_norm_bwd(const void* dy, const void* x, const void* w, const f
   using bf = __nv_bfloat16;
   const int nb = fm_norm_bwd_blocks(T);
   const int nvec = H / 8;
-  auto launch = [&](auto layer_norm, auto rms_norm) {
-    auto kernel = kind == 0 ? layer_norm : rms_norm;
+  // RMSNorm has no bias of its own; a caller that asks for the gradient of one all the same gets it
+  const bool bias = kind == 0 || db != nullptr;
+  auto launch = [&](auto layer_norm, auto rms_norm, auto rms_norm_bias) {
+    auto kernel = kind == 0 ? layer_norm : bias ? rms_norm_bias : rms_norm;
     kernel<<<nb, fm::kNormThreads, 0, s>>>((const bf*)dy, (const bf*)x, (const bf*)w, mean, rstd,
                                            (const bf*)res_grad, (bf*)dx, partial, T, H);
   };
-  if (nvec <= fm::kNormThreads) launch(fm::norm_bwd_kernel<1, true>, fm::norm_bwd_kernel<1, false>);
-  else if (nvec <= 2 * fm::kNormThreads) launch(fm::norm_bwd_kernel<2, true>, fm::norm_bwd_kernel<2, false>);
-  else launch(fm::norm_bwd_kernel<4, true>, fm::norm_bwd_kernel<4, false>);
+#define FM_NORM_BWD(C) \
+  launch(fm::norm_bwd_kernel<C, true, true>, fm::norm_bwd_kernel<C, false, false>, fm::norm_bwd_kernel<C, false, true>)
+  if (nvec <= fm::kNormThreads) FM_NORM_BWD(1);
+  else if (nvec <= 2 * fm::kNormThreads) FM_NORM_BWD(2);
+  else FM_NORM_BWD(4);
+#undef FM_NORM_BWD
   int rc = check_launch("norm_bwd");
   if (rc) return rc;
-  const int cols = kind == 0 ? 2 * H : H;
+  const int cols = bias ? 2 * H : H;
   fm::norm_bwd_reduce_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(partial, dw, db, nb, cols, H);
   return check_launch("norm_bwd_reduce");
 }

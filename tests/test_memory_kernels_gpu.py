@@ -147,3 +147,15 @@ def test_norm_forward(T, H, kind):
     assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * ref.abs().max()).all()
     assert ((rstd.double() - r.squeeze(1)).abs() <= 1e-5 * r.squeeze(1)).all()
     assert mean is None or ((mean.double() - mu.squeeze(1)).abs() <= 1e-5).all()
+
+
+@pytest.mark.parametrize("H", [520, 4096, 8192])
+def test_rms_norm_backward_with_a_bias_gradient(H):
+    """RMSNorm has no bias, but the call returns the column sums of dy when asked for a bias gradient."""
+    torch.manual_seed(H)
+    x, dy, w = _rand(300, H), _rand(300, H), _rand(H)
+    _, _, rstd = norm.norm_fwd(x, w, None, 1e-5, "rmsnorm")
+    dx, dw, db = norm.norm_bwd(dy, x, w, None, rstd, "rmsnorm", True)
+    dx2, dw2, none = norm.norm_bwd(dy, x, w, None, rstd, "rmsnorm", False)
+    assert none is None and torch.equal(dx, dx2) and torch.equal(dw, dw2)
+    assert ((db.double() - dy.double().sum(0)).abs() <= 2e-6 * dy.double().abs().sum(0) + 1e-6).all()
