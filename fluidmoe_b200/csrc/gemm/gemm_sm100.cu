@@ -330,10 +330,11 @@ struct EpiStore {
             const int col = t.n_tile * BN + c * 32;
             if (col >= a.N) break;
             if (residual != nullptr && col + 64 <= a.N) {
-              // The stage that turns the rows of the residual over to the lanes lies over the boxes.
+              // The stage that turns the rows of the residual over to the lanes lies over both boxes, so nothing
+              // may be on its way; the block still takes the next box, so that the cut last block, which opens its
+              // own with one store pending, does not get the one that this store reads.
               uint32_t w[32];
-              if (lane == 0) bulk_wait_group_read<0>();
-              __syncwarp();
+              uint8_t* box = bs.next<0>();
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
                 float v[32], p[32];
@@ -344,7 +345,6 @@ struct EpiStore {
                   w[16 * h + i] = pack_bf16x2(fmaf(v[2 * i], alpha, p[2 * i]), fmaf(v[2 * i + 1], alpha, p[2 * i + 1]));
               }
               __syncwarp();
-              uint8_t* box = bs.stg;
 #pragma unroll
               for (int i = 0; i < 8; ++i) bs.put(box, i, make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]));
               bs.send(maps, box, col, (int)row0, z);

@@ -421,3 +421,30 @@ def test_residual_and_device_scalar(M, N, K, how, cta_pair, monkeypatch):
     if g is not None:
         want = 0.375 * a.double().sum(0)[:, None].expand(K, 72)
         assert ((g[0].double() - want).abs() <= 1e-5 * a.double().abs().sum(0)[:, None]).all()
+
+
+@pytest.mark.parametrize("N", [200, 328, 1000])
+@pytest.mark.parametrize("in_place", [False, True])
+@pytest.mark.parametrize("cta_pair", [0, 1])
+def test_residual_store_with_a_cut_last_block(N, in_place, cta_pair, monkeypatch):
+    """A warp that stores a whole 64-column block and then the cut last one (N mod 128 between 64 and 128): the
+    second must not refill the box that the first store still reads.  Rows enough for every SM to store at
+    once; every element against 64 bits, and the same bytes each time."""
+    monkeypatch.setattr(gemm, "CTA_PAIR", cta_pair)
+    torch.manual_seed(N)
+    M, K = 40_000, 64
+    a, w, r = _rand(M, K), _rand(N, K), _rand(M, N)
+    ref = a.double() @ w.double().t() + r.double()
+    first = None
+    for _ in range(8):
+        if in_place:
+            out = gemm.grouped_gemm(a, w, b_layout="nk", out=r.clone(), accumulate=True)
+        else:
+            out = gemm.grouped_gemm(a, w, b_layout="nk", residual=r)
+        if first is None:
+            first = out
+            # fp32 sums of K products, then one rounding: 2^-8 of the value
+            assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * K ** 0.5).all()
+        assert torch.equal(out, first)
+    torch.cuda.synchronize()
+    gemm.check_status()
