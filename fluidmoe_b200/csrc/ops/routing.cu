@@ -242,13 +242,15 @@ moe_plan_kernel(const long long* __restrict__ top_idx, const float* __restrict__
   count = __reduce_add_sync(0xffffffffu, digit_s[0][lane][0]);
   if (__reduce_add_sync(0xffffffffu, digit_s[0][lane][1]) != count) {
     // Some token names this expert twice (a replayed routing may): its first choice counts, and the
-    // pass above kept either.
+    // pass above kept either.  The others have no slot.
     for (int t = lo; t < hi; ++t) {
       if (choice_s[plan_pos(t)] == 255) continue;
       int j = 0;
       while ((int)top_idx[(long long)t * k + j] != e) ++j;
       choice_s[plan_pos(t)] = (uint8_t)j;
       bits_s[plan_pos(t)] = __float_as_uint(top_probs[(long long)t * k + j]);
+      for (++j; j < k; ++j)
+        if ((int)top_idx[(long long)t * k + j] == e) slot_of_token[(long long)t * k + j] = -1;
     }
   }
   const int kept_total = min(count, cap);
@@ -464,6 +466,9 @@ moe_plan_large_kernel(const long long* __restrict__ top_idx, const float* __rest
       if (kept) slot_of_token[(long long)t * k + j] = (int)slot;
     }
     if (routed && !kept) slot_of_token[(long long)t * k + j] = -1;
+    if (routed)
+      for (int i = j + 1; i < k; ++i)      // a token that names this expert again has no slot for it
+        if ((int)top_idx[(long long)t * k + i] == e) slot_of_token[(long long)t * k + i] = -1;
   }
   if (tid == 0) {
     routed_per_expert[e] = kept_total;

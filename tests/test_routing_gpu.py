@@ -95,6 +95,32 @@ def test_padded_plan_counts_a_repeated_choice_once():
     assert got.permuted_probs.tolist() == [0.75, 0.5, 0.625, 0.5, 0.375, 0.875]
 
 
+@pytest.mark.parametrize("T", [4, 1000, 50_000])     # the last takes the kernel for rows beyond shared memory
+@pytest.mark.parametrize("k", [2, 5])
+def test_padded_plan_gives_repeated_choices_no_slot(T, k):
+    """Every entry of ``slot_of_token`` is written: the slot of a kept first choice, -1 for a dropped one and for
+    every later choice of the same expert (the un-permute takes any value from 0 up as a row)."""
+    E = 3
+    g = torch.Generator().manual_seed(T)
+    idx = torch.randint(0, E, (T, k), generator=g)
+    probs = torch.rand(T, k, generator=g) + 0.01
+    cap = max(1, T // 2)
+    # blocks of the plan's sizes, filled and given back, so that what a kernel leaves out shows
+    filled = [torch.full((T, k), 7, dtype=torch.int32, device="cuda") for _ in range(4)]
+    del filled
+    got = router.build_padded_plan(idx.cuda(), probs.cuda(), E, cap)
+    slot, tok = got.slot_of_token.cpu().long(), got.sorted_indices.cpu()
+    first = torch.ones(T, k, dtype=torch.bool)
+    for j in range(1, k):
+        first[:, j] = (idx[:, :j] != idx[:, j:j + 1]).all(1)
+    assert (slot[~first] == -1).all()
+    kept = slot >= 0
+    assert torch.equal(tok[slot[kept]], torch.arange(T)[:, None].expand(T, k)[kept])
+    assert torch.equal(slot[kept] // cap, idx[kept])
+    assert torch.equal(got.permuted_probs.cpu()[slot[kept]], probs[kept])
+    assert torch.bincount(idx[kept], minlength=E).tolist() == got.routed_per_expert.tolist()
+
+
 @pytest.mark.parametrize("T,E,k,skew", [(1, 1, 1, 0.0), (1, 8, 2, 0.0), (63, 8, 2, 3.0), (64, 1, 1, 0.0),
                                         (683, 64, 6, 0.1), (1531, 64, 6, 0.05), (4096, 8, 2, 0.0), (4097, 1024, 8, 0.0)])
 def test_dropless_plan_local(T, E, k, skew):
