@@ -507,18 +507,25 @@ unpermute_reduce_kernel(const __nv_bfloat16* __restrict__ rows, const int* __res
 // --------------------------------------------------------------------------------------------
 // Embedding gradient: main[ids[t]] += dy[t], one 16-byte piece of a bf16 row per thread, added to the fp32
 // row with two four-wide reductions.  Converting to fp32 first and adding element by element took 163 us
-// for 4096 tokens of 4096 columns, this takes 29.
+// for 4096 tokens of 4096 columns, this takes 29.  An id that is no row of the table is left out and reported.
 // --------------------------------------------------------------------------------------------
+constexpr int kKernelIdEmbeddingGrad = 18;
+
 __global__ void __launch_bounds__(256)
 embedding_grad_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ dy,
-                      float* __restrict__ main_grad, long long total, int nvec) {
+                      float* __restrict__ main_grad, long long total, int nvec, long long rows, int* status) {
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     const long long t = idx / nvec;
     const int i = (int)(idx - t * nvec);
+    const long long id = ids[t];
+    if (id < 0 || id >= rows) {
+      if (i == 0) report_status(status, kStatusBadArgs, kKernelIdEmbeddingGrad, (int)t, (int)rows, (int)id);
+      continue;
+    }
     float v[8];
     unpack8(reinterpret_cast<const uint4*>(dy)[idx], v);
-    float* dst = main_grad + (ids[t] * nvec + i) * 8;
+    float* dst = main_grad + (id * nvec + i) * 8;
     red_add_v4_f32(dst, v[0], v[1], v[2], v[3]);
     red_add_v4_f32(dst + 4, v[4], v[5], v[6], v[7]);
   }
@@ -1062,8 +1069,8 @@ extern "C" int fm_adam_multi(const FmAdamTensor* tensors, int count, float lr, f
   return check_launch("adam_multi");
 }
 
-extern "C" int fm_embedding_grad(const long long* ids, const void* dy, float* main_grad, int T, int H,
-                                 cudaStream_t s) {
+extern "C" int fm_embedding_grad(const long long* ids, const void* dy, float* main_grad, int T, int H, long long rows,
+                                 int* status, cudaStream_t s) {
   if (H % 8 != 0 || (reinterpret_cast<uintptr_t>(dy) & 15) || (reinterpret_cast<uintptr_t>(main_grad) & 15)) {
     fm_set_error("embedding_grad: H must be a multiple of 8 and rows 16-byte aligned");
     return -1;
@@ -1071,7 +1078,7 @@ extern "C" int fm_embedding_grad(const long long* ids, const void* dy, float* ma
   const long long total = (long long)T * (H / 8);
   if (total == 0) return 0;
   fm::embedding_grad_kernel<<<grid_for(total, 256), 256, 0, s>>>(ids, (const __nv_bfloat16*)dy, main_grad, total,
-                                                                H / 8);
+                                                                H / 8, rows, status);
   return check_launch("embedding_grad");
 }
 

@@ -73,9 +73,9 @@ void bind_ops(py::module_& m) {
     chk(fm_router_wgrad(p<const void*>(x), p<const float*>(dl), p<float*>(partial), p<float*>(dw), T, H, E, st(s)),
         "router_wgrad");
   });
-  m.def("embedding_grad", [](u ids, u dy, u main_grad, int T, int H, u s) {
-    chk(fm_embedding_grad(p<const long long*>(ids), p<const void*>(dy), p<float*>(main_grad), T, H, st(s)),
-        "embedding_grad");
+  m.def("embedding_grad", [](u ids, u dy, u main_grad, int T, int H, long long rows, u status, u s) {
+    chk(fm_embedding_grad(p<const long long*>(ids), p<const void*>(dy), p<float*>(main_grad), T, H, rows,
+                          p<int*>(status), st(s)), "embedding_grad");
   });
   // tensors: (parameter, gradient, first moment, second moment, elements) per entry
   m.def("adam_multi", [](const std::vector<std::tuple<u, u, u, u, long long>>& tensors, float lr, float b1, float b2,

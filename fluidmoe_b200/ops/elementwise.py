@@ -219,14 +219,21 @@ def router_wgrad(x, dlogits):
 
 
 def embedding_grad_(main, ids, dy) -> bool:
-    """``main[ids[t]] += dy[t]`` in place (fp32 rows, bf16 gradients); False when the kernel does not take these."""
-    if not (main.is_cuda and dy.is_cuda and ids.is_cuda) or main.dtype != torch.float32 or dy.dtype != torch.bfloat16 \
-            or ids.dtype != torch.int64 or main.shape[1] % 8 or not main.is_contiguous() or main.data_ptr() % 16:
+    """``main[ids[t]] += dy[t]`` in place (fp32 rows, bf16 gradients); False when the kernel does not take these,
+    or when sums in a fixed order are asked for (the kernel adds with atomics).  An id that is no row of
+    ``main`` is left out and reported through ``gemm.check_status``."""
+    if not (main.is_cuda and main.device == dy.device == ids.device) or main.dtype != torch.float32 \
+            or dy.dtype != torch.bfloat16 or ids.dtype != torch.int64 or main.shape[1] % 8 \
+            or not main.is_contiguous() or main.data_ptr() % 16:
+        return False
+    if ids.dim() != 1 or tuple(dy.shape) != (ids.numel(), main.shape[1]) or torch.are_deterministic_algorithms_enabled():
         return False
     dy, ids = dy.contiguous(), ids.contiguous()
     if dy.data_ptr() % 16:
         return False
-    _native.lib().embedding_grad(ids.data_ptr(), dy.data_ptr(), main.data_ptr(), dy.shape[0], dy.shape[1], _s())
+    from .gemm import status_buffer
+    _native.lib().embedding_grad(ids.data_ptr(), dy.data_ptr(), main.data_ptr(), dy.shape[0], dy.shape[1],
+                                 main.shape[0], status_buffer(main.device).data_ptr(), _s())
     return True
 
 

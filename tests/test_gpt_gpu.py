@@ -47,3 +47,32 @@ def test_embedding_backward_on_gpu_adds_rows_into_main_grad():
     ref = torch.zeros(V, H, device=dev).index_add_(0, ids.reshape(-1), gy.reshape(-1, H).float())
     assert w.grad is None
     assert (w.main_grad - ref).abs().max().item() < 1e-3 * (ref.abs().max().item() + 1)
+
+
+@pytest.mark.parametrize("deterministic", [False, True])
+def test_embedding_gradient_takes_only_what_fits(deterministic):
+    """Shapes that do not belong together go to the general path, which refuses them; so does every call while
+    sums in a fixed order are asked for.  Ids that are no rows are left out and reported."""
+    from fluidmoe_b200.ops import elementwise, gemm
+    dev = torch.device("cuda", 0)
+    V, H, T = 40, 64, 24
+    dy = torch.randn(T, H, device=dev).bfloat16()
+    ids = torch.arange(T, device=dev) * 3 - 4          # -4, -1, 2, ..., 65: ids below and above the table
+    main = torch.zeros(V, H, device=dev)
+    assert not elementwise.embedding_grad_(main, ids[:-1], dy)
+    assert not elementwise.embedding_grad_(main, ids, dy[:, :32].contiguous())
+    assert not elementwise.embedding_grad_(main, ids, dy.cpu())
+    torch.use_deterministic_algorithms(deterministic)
+    try:
+        took = elementwise.embedding_grad_(main, ids, dy)
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert took != deterministic
+    ref = torch.zeros(V, H, device=dev)
+    if took:
+        with pytest.raises(gemm.FluidKernelTimeout, match="kernel 18 "):
+            gemm.check_status()
+        ok = (ids >= 0) & (ids < V)
+        ref[ids[ok]] = dy[ok].float()
+    gemm.check_status()
+    assert torch.equal(main, ref)
