@@ -131,7 +131,7 @@ class FusedAdam:
             self._pending_events.clear()
         self.step_count += 1
         b1, b2 = self.betas
-        batches = {}      # device -> tensors that one launch updates
+        batches = {}      # device -> parameter address -> tensors that one launch updates
         for p in self.params:
             if getattr(p, "_fused_update_done", False):
                 p._fused_update_done = False      # updated by its weight-gradient GEMM already
@@ -146,7 +146,11 @@ class FusedAdam:
                 # a parameter whose update takes longer than a launch keeps a launch of its own: the kernel for
                 # one tensor streams 131 M elements in 489 us, the one for many in 526
                 if st["master"] is None and st["m"].dtype == self.state_dtype and p.numel() < 1 << 22:
-                    batches.setdefault(p.device, []).append((p.data, g, st["m"], st["v"]))
+                    batch = batches.setdefault(p.device, {})
+                    if p.data_ptr() in batch:       # tied parameters take their updates one after the other
+                        self._update_together(batch.values(), grad_scale)
+                        batch.clear()
+                    batch[p.data_ptr()] = (p.data, g, st["m"], st["v"])
                 else:
                     elementwise.adam_step(p.data, st["master"], g, st["m"], st["v"], self.lr, b1, b2, self.eps,
                                           self.weight_decay, self.step_count, grad_scale)
@@ -163,10 +167,14 @@ class FusedAdam:
             if st["master"] is not None:
                 st["master"].copy_(w)
             p.data.copy_(w.to(p.dtype))
-        for tensors in batches.values():
-            from . import elementwise
-            elementwise.adam_multi(tensors, self.state_dtype == torch.bfloat16, self.lr, b1, b2, self.eps,
-                                   self.weight_decay, self.step_count, grad_scale)
+        for batch in batches.values():
+            self._update_together(batch.values(), grad_scale)
+
+    def _update_together(self, tensors, grad_scale: float) -> None:
+        """One launch over ``(p, g, m, v)`` of different parameters on one device."""
+        from . import elementwise
+        elementwise.adam_multi(list(tensors), self.state_dtype == torch.bfloat16, self.lr, *self.betas, self.eps,
+                               self.weight_decay, self.step_count, grad_scale)
 
     def zero_grad(self, set_to_none: bool = True) -> None:
         for p in self.params:

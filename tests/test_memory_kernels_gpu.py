@@ -159,3 +159,23 @@ def test_rms_norm_backward_with_a_bias_gradient(H):
     dx2, dw2, none = norm.norm_bwd(dy, x, w, None, rstd, "rmsnorm", False)
     assert none is None and torch.equal(dx, dx2) and torch.equal(dw, dw2)
     assert ((db.double() - dy.double().sum(0)).abs() <= 2e-6 * dy.double().abs().sum(0) + 1e-6).all()
+
+
+def test_adam_updates_tied_parameters_one_after_the_other():
+    """A parameter that is listed twice, and two parameters over one array (moments of their own each)."""
+    from fluidmoe_b200.ops import elementwise
+    from fluidmoe_b200.ops.optim import FusedAdam
+    torch.manual_seed(9)
+    n, hyper = 100_000, dict(lr=1e-2, weight_decay=0.1)
+    w, w0, g, g2 = _rand(n), _rand(n), torch.randn(n, device="cuda"), torch.randn(n, device="cuda")
+    w.copy_(w0)
+    p, tied, other = torch.nn.Parameter(w), torch.nn.Parameter(w), torch.nn.Parameter(_rand(64))
+    p.main_grad, tied.main_grad, other.main_grad = g, g2, torch.randn(64, device="cuda")
+    opt = FusedAdam([p, other, tied, p], **hyper)
+    opt.step()
+    m, v, m2, v2 = (torch.zeros(n, device="cuda") for _ in range(4))
+    for grad, a, b in ((g, m, v), (g2, m2, v2), (g, m, v)):
+        elementwise.adam_multi([(w0, grad, a, b)], False, hyper["lr"], 0.9, 0.999, 1e-8, hyper["weight_decay"], 1)
+    assert torch.equal(w, w0)
+    for q, a, b in ((p, m, v), (tied, m2, v2)):
+        assert torch.equal(opt.state[id(q)]["m"], a) and torch.equal(opt.state[id(q)]["v"], b)
