@@ -143,8 +143,9 @@ class FusedAdam:
             if p.is_cuda and p.dtype == torch.bfloat16 and g.dtype == torch.float32 and _native.available() \
                     and p.is_contiguous() and g.is_contiguous():
                 from . import elementwise
-                # a parameter whose update takes longer than a launch keeps a launch of its own: the kernel for
-                # one tensor streams 131 M elements in 489 us, the one for many in 526
+                # a parameter whose update takes longer than a launch keeps a launch of its own.  Four tensors with
+                # fp32 moments, a launch each against one for all: 1 M elements 16.9 and 11.7 us, 4 M 73 and 68, 8 M
+                # 134 and 132, 16 M 254 and 261, 32 M 499 and 536: the line lies where sharing no longer gives anything
                 if st["master"] is None and st["m"].dtype == self.state_dtype and p.numel() < 1 << 22:
                     batch = batches.setdefault(p.device, {})
                     if p.data_ptr() in batch:       # tied parameters take their updates one after the other
@@ -171,9 +172,17 @@ class FusedAdam:
             self._update_together(batch.values(), grad_scale)
 
     def _update_together(self, tensors, grad_scale: float) -> None:
-        """One launch over ``(p, g, m, v)`` of different parameters on one device."""
+        """One launch over ``(p, g, m, v)`` of different parameters on one device.  A tensor that is alone takes the
+        kernel for one: its small pieces of work fill the chip (65536 elements 2.5 us against 4.8, a million
+        4.5 against 5.0)."""
         from . import elementwise
-        elementwise.adam_multi(list(tensors), self.state_dtype == torch.bfloat16, self.lr, *self.betas, self.eps,
+        tensors = list(tensors)
+        if len(tensors) == 1:
+            p, g, m, v = tensors[0]
+            elementwise.adam_step(p, None, g, m, v, self.lr, *self.betas, self.eps, self.weight_decay, self.step_count,
+                                  grad_scale)
+            return
+        elementwise.adam_multi(tensors, self.state_dtype == torch.bfloat16, self.lr, *self.betas, self.eps,
                                self.weight_decay, self.step_count, grad_scale)
 
     def zero_grad(self, set_to_none: bool = True) -> None:

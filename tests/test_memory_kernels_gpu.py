@@ -169,9 +169,11 @@ def test_adam_updates_tied_parameters_one_after_the_other():
     n, hyper = 100_000, dict(lr=1e-2, weight_decay=0.1)
     w, w0, g, g2 = _rand(n), _rand(n), torch.randn(n, device="cuda"), torch.randn(n, device="cuda")
     w.copy_(w0)
-    p, tied, other = torch.nn.Parameter(w), torch.nn.Parameter(w), torch.nn.Parameter(_rand(64))
-    p.main_grad, tied.main_grad, other.main_grad = g, g2, torch.randn(64, device="cuda")
-    opt = FusedAdam([p, other, tied, p], **hyper)
+    p, tied, others = torch.nn.Parameter(w), torch.nn.Parameter(w), [torch.nn.Parameter(_rand(64)) for _ in range(3)]
+    p.main_grad, tied.main_grad = g, g2
+    for o in others:
+        o.main_grad = torch.randn(64, device="cuda")
+    opt = FusedAdam([p, others[0], tied, others[1], p, others[2]], **hyper)
     opt.step()
     m, v, m2, v2 = (torch.zeros(n, device="cuda") for _ in range(4))
     for grad, a, b in ((g, m, v), (g2, m2, v2), (g, m, v)):
@@ -179,3 +181,23 @@ def test_adam_updates_tied_parameters_one_after_the_other():
     assert torch.equal(w, w0)
     for q, a, b in ((p, m, v), (tied, m2, v2)):
         assert torch.equal(opt.state[id(q)]["m"], a) and torch.equal(opt.state[id(q)]["v"], b)
+
+
+@pytest.mark.parametrize("count", [1, 2])
+def test_adam_of_one_tensor_takes_the_kernel_for_one(count, monkeypatch):
+    from fluidmoe_b200.ops import elementwise
+    from fluidmoe_b200.ops.optim import FusedAdam
+    calls = []
+    for name in ("adam_step", "adam_multi"):
+        real = getattr(elementwise, name)
+        monkeypatch.setattr(elementwise, name, lambda *a, _n=name, _f=real, **kw: (calls.append(_n), _f(*a, **kw)))
+    params = [torch.nn.Parameter(_rand(1000 + i)) for i in range(count)]
+    start = [p.detach().double() for p in params]
+    for p in params:      # gradients well above eps
+        p.main_grad = torch.where(torch.rand(p.shape, device="cuda") < 0.5, -1.0, 1.0) * (torch.rand(p.shape, device="cuda") + 0.1)
+    FusedAdam(params, lr=1e-2, weight_decay=0.1).step()
+    assert calls == (["adam_step"] if count == 1 else ["adam_multi"])
+    for p, s in zip(params, start):
+        # the first step moves a weight by lr * (sign of the gradient + decay), then one rounding of bf16
+        ref = s - 1e-2 * (torch.sign(p.main_grad.double()) + 0.1 * s)
+        assert ((p.detach().double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all()
