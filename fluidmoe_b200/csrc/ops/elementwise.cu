@@ -378,8 +378,8 @@ norm_bwd_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw
 // --------------------------------------------------------------------------------------------
 constexpr int kKernelIdRopeWait = 16;
 __global__ void rope_packed_kernel(__nv_bfloat16* __restrict__ t, const float* __restrict__ freqs,
-                                   long long rows, int heads_per_row, int rope_heads, int d,
-                                   int rot, int rows_per_pos, int backward, const int* wait_flags,
+                                   long long rows, int heads_per_row, int rope_heads, int heads_per_cta,
+                                   int d, int rot, int rows_per_pos, int backward, const int* wait_flags,
                                    int wait_n, int wait_expected, unsigned long long* wait_ns,
                                    unsigned long long timeout_ns, int* status) {
   // first consumer of the projection buffer that peers fill: wait for their rows here
@@ -395,9 +395,9 @@ __global__ void rope_packed_kernel(__nv_bfloat16* __restrict__ t, const float* _
     const long long pos = row / rows_per_pos;
     // `freqs` holds (cos, sin) pairs of the angles, [position][rot][2]: the table is computed once
     // per sequence on the host side instead of two sincosf per value here (which made the kernel
-    // compute-bound at 0.41 of the copy bandwidth), and read once for all heads of a row: 128 bytes of it
-    // for every 64 bytes of a head took 30 us for 4096 positions of 8 x (4 + 1) heads, once a
-    // row 18.
+    // compute-bound at 0.41 of the copy bandwidth), and read once for the heads that a thread takes: 128 bytes of
+    // it for every 64 bytes of a head took 25 us for 4096 positions of 8 x (4 + 1) heads, once a
+    // row 14.
     const float4* f1 = reinterpret_cast<const float4*>(freqs + (pos * rot + vi * 8) * 2);
     const float4* f2 = reinterpret_cast<const float4*>(freqs + (pos * rot + half + vi * 8) * 2);
     float4 t1[4], t2[4];      // cos, sin of two neighbours each
@@ -406,9 +406,10 @@ __global__ void rope_packed_kernel(__nv_bfloat16* __restrict__ t, const float* _
       t1[j] = f1[j];
       t2[j] = f2[j];
     }
-    __nv_bfloat16* base = t + row * heads_per_row * d + vi * 8;
+    const int h0 = blockIdx.y * heads_per_cta, h1 = min(rope_heads, h0 + heads_per_cta);
+    __nv_bfloat16* base = t + (row * heads_per_row + h0) * d + vi * 8;
 #pragma unroll 4
-    for (int h = 0; h < rope_heads; ++h, base += d) {
+    for (int h = h0; h < h1; ++h, base += d) {
       uint4* p1 = reinterpret_cast<uint4*>(base);
       uint4* p2 = reinterpret_cast<uint4*>(base + half);
       float a[8], b[8], o1[8], o2[8];
@@ -952,8 +953,18 @@ extern "C" int fm_rope_packed_gated(void* t, const float* freqs, long long rows,
     return -1;
   }
   const long long total = rows * (rot / 16);
-  fm::rope_packed_kernel<<<grid_for(total, 256), 256, 0, s>>>(
-      (__nv_bfloat16*)t, freqs, rows, heads_per_row, rope_heads, d, rot, rows_per_pos, backward, wait_flags,
+  // A thread takes all heads of its piece of a row, so that the table is read once for them, as long as that gives
+  // every SM a CTA; with fewer rows the heads are split.  One KV head and 32 query heads, 64 positions: 12.6 us
+  // with all heads in one thread, 2.9 split (one head a thread in every case: 3.0); 512: 12.6, 4.0 (5.0); 4096: 13.5, 10.0
+  // (21.5); 64 positions of 8 x (4 + 1) heads: 4.0, 2.7 (2.9).
+  const long long pieces = total > 0 ? total : 1;
+  long long splits = (148 * 256 + pieces - 1) / pieces;
+  if (splits > rope_heads) splits = rope_heads;
+  if (splits < 1) splits = 1;
+  const int per = (int)((rope_heads + splits - 1) / splits);
+  const dim3 grid(grid_for(total, 256), per > 0 ? (rope_heads + per - 1) / per : 1);
+  fm::rope_packed_kernel<<<grid, 256, 0, s>>>(
+      (__nv_bfloat16*)t, freqs, rows, heads_per_row, rope_heads, per, d, rot, rows_per_pos, backward, wait_flags,
       wait_n, wait_expected, wait_ns, timeout_ns ? timeout_ns : 4000000000ull, status);
   return check_launch("rope_packed");
 }

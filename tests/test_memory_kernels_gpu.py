@@ -201,3 +201,21 @@ def test_adam_of_one_tensor_takes_the_kernel_for_one(count, monkeypatch):
         # the first step moves a weight by lr * (sign of the gradient + decay), then one rounding of bf16
         ref = s - 1e-2 * (torch.sign(p.main_grad.double()) + 0.1 * s)
         assert ((p.detach().double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all()
+
+
+@pytest.mark.parametrize("s,G,qpg,d,rot", [(1, 1, 32, 128, 128), (64, 1, 32, 128, 128), (300, 1, 7, 128, 64), (590, 2, 32, 64, 64),
+                                           (595, 1, 70, 128, 128), (64, 8, 4, 128, 128), (4700, 1, 2, 128, 128)])
+@pytest.mark.parametrize("backward", [False, True])
+def test_rope_with_the_heads_split_over_threads(s, G, qpg, d, rot, backward):
+    """Few rows and many heads: each head once, also where the split does not divide them; the same bytes as with
+    every group as a tensor of its own."""
+    from fluidmoe_b200.ops import rope
+    torch.manual_seed(s)
+    x, f = _rand(s, 1, G, qpg + 2, d), torch.randn(s, 1, 1, rot, device="cuda")
+    got = rope.rope_packed_(x.clone().view(s, 1, G, -1), f, qpg, d, backward=backward).view_as(x)
+    for h in range(qpg + 1):
+        # one rotated head and a value head
+        one = torch.cat((x[:, :, :, h:h + 1], x[:, :, :, h:h + 1], x[:, :, :, -1:]), 3).contiguous()
+        ref = rope.rope_packed_(one.view(s, 1, G, -1), f, 1, d, backward=backward).view_as(one)
+        assert torch.equal(got[:, :, :, h], ref[:, :, :, 0])
+    assert torch.equal(got[:, :, :, -1], x[:, :, :, -1])
