@@ -137,9 +137,20 @@ def router_dgrad(dlogits: torch.Tensor, router_weight: torch.Tensor, dtype: torc
     return (d @ w.t()).to(dtype)
 
 
+def _wgrad_kernel_pays(T: int, H: int, E: int) -> bool:
+    """Where the kernel for the router weight gradient is faster than a conversion of ``x`` and the library's
+    product (us, library and kernel).  Few tokens leave its CTAs a chain of loads each: 64 tokens, 4096 x 16, 7.8 and
+    11.6; 256 11.5 and 11.9; 512 17.6 and 12.6.  Many experts read ``x`` again for every 16 of them: 4096 tokens of
+    4096 columns, 64 experts 116 and 78, 128 151 and 145, 256 209 and 319; with narrow rows that costs less: 1024
+    columns, 128 experts 62 and 45."""
+    if E <= 8:
+        return T >= 128
+    return T >= 512 and (E <= 32 or (E <= 64 and T >= 1024) or (E <= 160 and H * E <= 1 << 17))
+
+
 def router_wgrad(x: torch.Tensor, dlogits: torch.Tensor) -> torch.Tensor:
     """Router weight gradient ``x[T, H]^T @ dlogits[T, E]`` in fp32."""
-    if _native.use_native(x, dlogits):
+    if _native.use_native(x, dlogits) and _wgrad_kernel_pays(x.shape[0], x.shape[1], dlogits.shape[1]):
         from . import elementwise
         res = elementwise.router_wgrad(x, dlogits)
         if res is not None:

@@ -219,3 +219,33 @@ def test_rope_with_the_heads_split_over_threads(s, G, qpg, d, rot, backward):
         ref = rope.rope_packed_(one.view(s, 1, G, -1), f, 1, d, backward=backward).view_as(one)
         assert torch.equal(got[:, :, :, h], ref[:, :, :, 0])
     assert torch.equal(got[:, :, :, -1], x[:, :, :, -1])
+
+
+@pytest.mark.parametrize("T", [1, 31, 33, 1531])
+@pytest.mark.parametrize("H,E", [(4, 1), (2, 3), (264, 8), (512, 16), (520, 17), (1028, 64), (2048, 70)])
+def test_router_weight_gradient_kernel(T, H, E):
+    """The kernel itself, also at the sizes that ``ops.router`` leaves to the library."""
+    from fluidmoe_b200.ops import elementwise
+    torch.manual_seed(T + E)
+    x, dl = _rand(T, H), torch.randn(T, E, device="cuda")
+    got = elementwise.router_wgrad(x, dl)
+    assert (got is None) == (H % 4 != 0)
+    if got is not None:
+        ref, terms = x.double().t() @ dl.double(), x.double().abs().t() @ dl.double().abs()
+        # fp32 sums of T terms, a few hundred at a time
+        assert ((got.double() - ref).abs() <= 2e-6 * terms).all()
+
+
+@pytest.mark.parametrize("T,H,E,kernel", [(127, 64, 8, False), (128, 64, 8, True), (511, 512, 32, False), (512, 512, 32, True),
+                                          (512, 2048, 64, True), (512, 2056, 64, False), (1024, 2056, 64, True),
+                                          (600, 1024, 128, True), (600, 1032, 128, False), (600, 256, 161, False)])
+def test_router_weight_gradient_takes_the_kernel_where_it_pays(T, H, E, kernel):
+    from fluidmoe_b200.ops import elementwise, router
+    torch.manual_seed(T)
+    x, dl = _rand(T, H), torch.randn(T, E, device="cuda")
+    before = elementwise.LAUNCHES
+    got = router.router_wgrad(x, dl)
+    assert (elementwise.LAUNCHES > before) == kernel
+    ref, terms = x.double().t() @ dl.double(), x.double().abs().t() @ dl.double().abs()
+    # fp32 sums of T terms in either path: 2^-24 of their absolute sum a step, T steps at the worst, sqrt(T) as a rule
+    assert ((got.double() - ref).abs() <= 4 * T ** 0.5 * 2.0 ** -24 * terms).all()
