@@ -102,7 +102,8 @@ topk_softmax_warp_kernel(const float* __restrict__ logits, long long* __restrict
   }
 }
 
-// More than 256 experts: one thread per token.
+// One thread per token: more than 256 experts, or so many tokens with so few experts that a warp each is the
+// longer way (see fm_topk_softmax).
 __global__ void topk_softmax_kernel(const float* __restrict__ logits, long long* __restrict__ idx_out,
                                     float* __restrict__ prob_out, int T, int E, int k) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -715,11 +716,16 @@ extern "C" int fm_topk_softmax(const float* logits, long long* idx, float* probs
     return -1;
   }
   const int grid = (T + 7) / 8;
-  if (E <= 32) fm::topk_softmax_warp_kernel<1><<<grid, 256, 0, s>>>(logits, idx, probs, T, E, k);
+  // A warp per token costs the same for every E up to 32 and grows with T, a thread per token costs E * k
+  // comparisons in a row whatever T is, as long as the tokens find room side by side.  Warp and thread, us: 16384
+  // tokens, 8 experts, k = 2, 3.9 and 3.3, k = 4 4.8 and 5.8; 65536 tokens, 8 experts, k = 2, 10.6 and 4.3, k = 8 19.9
+  // and 17.5; 16 experts, k = 2, 10.6 and 8.3, k = 4 13.4 and 15.2.
+  const bool threads = E > 256 || (E <= 16 && (long long)E * k * 1024 <= T && E * k <= (E <= 8 ? 64 : 32));
+  if (threads) fm::topk_softmax_kernel<<<(T + 127) / 128, 128, 0, s>>>(logits, idx, probs, T, E, k);
+  else if (E <= 32) fm::topk_softmax_warp_kernel<1><<<grid, 256, 0, s>>>(logits, idx, probs, T, E, k);
   else if (E <= 64) fm::topk_softmax_warp_kernel<2><<<grid, 256, 0, s>>>(logits, idx, probs, T, E, k);
   else if (E <= 128) fm::topk_softmax_warp_kernel<4><<<grid, 256, 0, s>>>(logits, idx, probs, T, E, k);
-  else if (E <= 256) fm::topk_softmax_warp_kernel<8><<<grid, 256, 0, s>>>(logits, idx, probs, T, E, k);
-  else fm::topk_softmax_kernel<<<(T + 127) / 128, 128, 0, s>>>(logits, idx, probs, T, E, k);
+  else fm::topk_softmax_warp_kernel<8><<<grid, 256, 0, s>>>(logits, idx, probs, T, E, k);
   return check_launch("topk_softmax");
 }
 

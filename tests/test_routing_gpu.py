@@ -48,6 +48,26 @@ def test_topk_softmax(E, k, kind):
     torch.testing.assert_close(probs.cpu().double(), ex / ex.sum(1, keepdim=True), rtol=1e-5, atol=1e-7, equal_nan=True)
 
 
+@pytest.mark.parametrize("E,k", [(1, 1), (2, 2), (7, 3), (8, 8), (9, 3), (16, 2)])
+@pytest.mark.parametrize("ties", [False, True])
+def test_topk_of_many_tokens_equals_that_of_few(E, k, ties):
+    """From 1024 * E * k tokens on a thread takes a token, below a warp; the same choices and, but for the order of
+    k terms, the same probabilities."""
+    T = 1024 * E * k
+    g = torch.Generator().manual_seed(E)
+    x = torch.randn(T, E, generator=g)
+    if ties:
+        x = torch.randint(-1, 2, (T, E), generator=g).float()
+        x[::5] = -math.inf
+        x[1::5, 0] = math.nan
+    x = x.cuda()
+    idx, probs = elementwise.topk_softmax(x, k)
+    for part in (slice(0, T // 2), slice(T // 2, T)):
+        i2, p2 = elementwise.topk_softmax(x[part], k)
+        assert torch.equal(idx[part], i2)
+        torch.testing.assert_close(probs[part], p2, rtol=2e-6, atol=0.0, equal_nan=True)
+
+
 def _routing(T, E, k, seed, skew=0.0):
     g = torch.Generator().manual_seed(seed)
     logits = torch.randn(T, E, generator=g) - skew * torch.arange(E)
