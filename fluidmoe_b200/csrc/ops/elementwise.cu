@@ -468,7 +468,10 @@ constexpr int kKernelIdUnpermuteWait = 15;
 // One thread per 16 bytes of a token, K known at compile time: the k rows and the residual are in flight
 // together, and a few tokens still fill the chip.  With one warp per token and a loop over k, 8192 tokens of
 // 2048 columns and k = 8 (336 MB) took 99 us, now 57; 64 tokens of 4096 columns and k = 2 17 us, now 6.
-template <int K>
+// More than eight choices go in rounds: sixteen rows in flight take 128 registers, which leaves too few threads.
+// 4096 tokens of 512 columns: k = 9 in one round 11.5 us (a warp per token 8.8), in two of six 8.0; k = 16 13.6 (15.6),
+// in four of four 9.6; 16384 tokens of 4096 columns, k = 9: 304 (329) and 259.
+template <int K, int kRounds>
 __global__ void __launch_bounds__(256)
 unpermute_reduce_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict__ slot,
                         const __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ out, int T, int k,
@@ -482,24 +485,27 @@ unpermute_reduce_kernel(const __nv_bfloat16* __restrict__ rows, const int* __res
        idx += (long long)gridDim.x * blockDim.x) {
     const long long t = total <= 0xffffffffll ? (long long)((unsigned)idx / nvec) : idx / nvec;
     const int i = (int)(idx - t * nvec);
-    uint4 v[K];
-    int sl[K];
-#pragma unroll
-    for (int j = 0; j < K; ++j) sl[j] = j < k ? slot[t * k + j] : -1;
     uint4 res = make_uint4(0, 0, 0, 0);
-    if (residual != nullptr) res = reinterpret_cast<const uint4*>(residual + t * H)[i];
-#pragma unroll
-    for (int j = 0; j < K; ++j)
-      if (sl[j] >= 0) v[j] = reinterpret_cast<const uint4*>(rows + (long long)sl[j] * H)[i];
     float acc[8];
-    unpack8(res, acc);
+#pragma unroll 1
+    for (int r = 0; r < kRounds; ++r) {
+      uint4 v[K];
+      int sl[K];
 #pragma unroll
-    for (int j = 0; j < K; ++j) {
-      if (sl[j] < 0) continue;
-      float x[8];
-      unpack8(v[j], x);
+      for (int j = 0; j < K; ++j) sl[j] = r * K + j < k ? slot[t * k + r * K + j] : -1;
+      if (r == 0 && residual != nullptr) res = reinterpret_cast<const uint4*>(residual + t * H)[i];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) acc[q] += x[q];
+      for (int j = 0; j < K; ++j)
+        if (sl[j] >= 0) v[j] = reinterpret_cast<const uint4*>(rows + (long long)sl[j] * H)[i];
+      if (r == 0) unpack8(res, acc);
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        if (sl[j] < 0) continue;
+        float x[8];
+        unpack8(v[j], x);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[q] += x[q];
+      }
     }
     reinterpret_cast<uint4*>(out + t * H)[i] = pack8(acc);
   }
@@ -998,12 +1004,13 @@ extern "C" int fm_unpermute_reduce_gated(const void* rows, const int* slot, cons
         (const __nv_bfloat16*)rows, slot, (const __nv_bfloat16*)residual, (__nv_bfloat16*)out, T, k, H, wait_flags,
         wait_n, wait_expected, wait_ns, timeout_ns ? timeout_ns : 4000000000ull, status);
   };
-  if (k <= 1) launch(fm::unpermute_reduce_kernel<1>);
-  else if (k <= 2) launch(fm::unpermute_reduce_kernel<2>);
-  else if (k <= 4) launch(fm::unpermute_reduce_kernel<4>);
-  else if (k <= 6) launch(fm::unpermute_reduce_kernel<6>);
-  else if (k <= 8) launch(fm::unpermute_reduce_kernel<8>);
-  else launch(fm::unpermute_reduce_kernel<16>);
+  if (k <= 1) launch(fm::unpermute_reduce_kernel<1, 1>);
+  else if (k <= 2) launch(fm::unpermute_reduce_kernel<2, 1>);
+  else if (k <= 4) launch(fm::unpermute_reduce_kernel<4, 1>);
+  else if (k <= 6) launch(fm::unpermute_reduce_kernel<6, 1>);
+  else if (k <= 8) launch(fm::unpermute_reduce_kernel<8, 1>);
+  else if (k <= 12) launch(fm::unpermute_reduce_kernel<6, 2>);
+  else launch(fm::unpermute_reduce_kernel<4, 4>);
   return check_launch("unpermute_reduce");
 }
 

@@ -249,3 +249,22 @@ def test_router_weight_gradient_takes_the_kernel_where_it_pays(T, H, E, kernel):
     ref, terms = x.double().t() @ dl.double(), x.double().abs().t() @ dl.double().abs()
     # fp32 sums of T terms in either path: 2^-24 of their absolute sum a step, T steps at the worst, sqrt(T) as a rule
     assert ((got.double() - ref).abs() <= 4 * T ** 0.5 * 2.0 ** -24 * terms).all()
+
+
+@pytest.mark.parametrize("k", [9, 10, 11, 12, 13, 14, 15, 16])
+@pytest.mark.parametrize("T,H", [(1, 8), (65, 72), (130, 2048)])
+@pytest.mark.parametrize("with_res", [False, True])
+def test_unpermute_in_rounds(k, T, H, with_res):
+    """More choices than one round holds: whole rounds, cut ones and choices without a row anywhere; the same
+    bytes as the loop over the choices gives."""
+    torch.manual_seed(k)
+    rows, res = _rand(T * k, H), _rand(T, H)
+    slot = torch.randperm(T * k, device="cuda").view(T, k).to(torch.int32)
+    slot[torch.rand(T, k, device="cuda") < 0.2] = -1
+    slot[::3, :8] = -1
+    got = permute.unpermute_reduce(rows, slot, res if with_res else None)
+    acc = res.float() if with_res else torch.zeros(T, H, device="cuda")
+    for j in range(k):
+        s = slot[:, j].long()
+        acc = torch.where((s >= 0)[:, None], acc + rows[s.clamp(min=0)].float(), acc)
+    assert torch.equal(got, acc.to(torch.bfloat16))
