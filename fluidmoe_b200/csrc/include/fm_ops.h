@@ -35,6 +35,8 @@ int fm_gather_rows(const void* x, const long long* idx, void* out, long long row
                    cudaStream_t s);
 int fm_unpermute_reduce(const void* rows, const int* slot, const void* residual, void* out, int T,
                         int k, int H, cudaStream_t s);
+// CTAs that it launches; `waits`: for the form that waits for peers.
+int fm_unpermute_grid(int T, int H, int waits);
 // The same, preceded by a bounded wait on `wait_n` per-source arrival counters (>= wait_expected).
 int fm_unpermute_reduce_gated(const void* rows, const int* slot, const void* residual, void* out, int T, int k,
                               int H, const int* wait_flags, int wait_n, int wait_expected,

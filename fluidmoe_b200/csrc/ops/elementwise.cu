@@ -991,6 +991,15 @@ extern "C" int fm_unpermute_reduce(const void* rows, const int* slot, const void
   return fm_unpermute_reduce_gated(rows, slot, residual, out, T, k, H, nullptr, 0, 0, nullptr, 0, nullptr, s);
 }
 
+// CTAs of an un-permute.  One that waits for rows of peers keeps its CTAs on the SMs until they are there: it gets no
+// more than one for eight tokens (4096 tokens of 4096 columns: 512 where a piece of 16 bytes per thread would make
+// 2368, all that fit on the chip at once), or one per SM, so that collectives, a background optimizer step or a
+// GEMM of another stream still find room beside it.
+extern "C" int fm_unpermute_grid(int T, int H, int waits) {
+  const int cap = waits ? grid_for(T, 8) : 148 * 16;
+  return grid_for((long long)T * (H / 8), 256, cap > 148 ? cap : 148);
+}
+
 extern "C" int fm_unpermute_reduce_gated(const void* rows, const int* slot, const void* residual,
                                          void* out, int T, int k, int H, const int* wait_flags, int wait_n,
                                          int wait_expected, unsigned long long* wait_ns,
@@ -1000,7 +1009,7 @@ extern "C" int fm_unpermute_reduce_gated(const void* rows, const int* slot, cons
     return -1;
   }
   auto launch = [&](auto kernel) {
-    kernel<<<grid_for((long long)T * (H / 8), 256), 256, 0, s>>>(
+    kernel<<<fm_unpermute_grid(T, H, wait_flags != nullptr), 256, 0, s>>>(
         (const __nv_bfloat16*)rows, slot, (const __nv_bfloat16*)residual, (__nv_bfloat16*)out, T, k, H, wait_flags,
         wait_n, wait_expected, wait_ns, timeout_ns ? timeout_ns : 4000000000ull, status);
   };

@@ -60,6 +60,7 @@ void bind_ops(py::module_& m) {
                                   H, p<const int*>(flags), n, expected, p<unsigned long long*>(wait_ns), timeout_ns,
                                   p<int*>(status), st(s)), "unpermute_reduce_gated");
   });
+  m.def("unpermute_grid", &fm_unpermute_grid);
   m.def("unpermute_reduce", [](u rows, u slot, u res, u out, int T, int k, int H, u s) {
     chk(fm_unpermute_reduce(p<const void*>(rows), p<const int*>(slot), p<const void*>(res),
                             p<void*>(out), T, k, H, st(s)), "unpermute_reduce");

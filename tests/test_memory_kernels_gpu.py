@@ -268,3 +268,20 @@ def test_unpermute_in_rounds(k, T, H, with_res):
         s = slot[:, j].long()
         acc = torch.where((s >= 0)[:, None], acc + rows[s.clamp(min=0)].float(), acc)
     assert torch.equal(got, acc.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("T", [1, 700, 5000, 20_000])
+@pytest.mark.parametrize("k", [2, 10])
+def test_waiting_unpermute_gives_the_same(T, k):
+    """The form that waits for peers, with counters that have arrived: its grid is smaller, so its threads take
+    several pieces each."""
+    from fluidmoe_b200.ops import elementwise, gemm
+    torch.manual_seed(T)
+    H = 512
+    rows, res = _rand(T * k, H), _rand(T, H)
+    slot = torch.randperm(T * k, device="cuda").view(T, k).to(torch.int32)
+    flags, waited = torch.full((2,), 5, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int64, device="cuda")
+    wait = dict(flags=flags.data_ptr(), n=2, expected=5, wait_ns=waited.data_ptr(), timeout_ns=1_000_000_000,
+                status=gemm.status_buffer(rows.device).data_ptr())
+    assert torch.equal(elementwise.unpermute_reduce(rows, slot, res, wait), elementwise.unpermute_reduce(rows, slot, res))
+    gemm.check_status()
