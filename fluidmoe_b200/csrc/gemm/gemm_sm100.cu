@@ -294,7 +294,7 @@ struct EpiStore {
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
                                       bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
-                                      volatile int* abort_flag) const {
+                                      volatile int* abort_flag, int kernel_id) const {
     const int lane = r & 31;
     const long long row = a.mode == 0 ? (long long)t.row_base + t.m0 + r : (long long)t.m0 + r;
     const long long row0 = row - lane;   // first row of this warp
@@ -578,7 +578,7 @@ struct EpiAdam {
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
                                       bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
-                                      volatile int* abort_flag) const {
+                                      volatile int* abort_flag, int kernel_id) const {
     constexpr int NB = BN / 64;          // 32-column blocks handled by this warp
     const int lane = r & 31;
     const long long row = a.mode == 0 ? (long long)t.row_base + t.m0 + r : (long long)t.m0 + r;
@@ -606,7 +606,7 @@ struct EpiAdam {
         }
         __syncwarp();
         if (!mbar_wait(wbar + (k & 1), (k >> 1) & 1, a.timeout_ns, abort_flag)) {
-          if (lane == 0) report_status(a.status, kStatusMbarTimeout, kKernelIdGemm2, 500 + k, 0, 0);
+          if (lane == 0) report_status(a.status, kStatusMbarTimeout, kernel_id, 500 + k, 0, 0);
           return;
         }
 #pragma unroll
@@ -746,7 +746,7 @@ struct EpiAct {
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
                                       bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
-                                      volatile int* abort_flag) const {
+                                      volatile int* abort_flag, int kernel_id) const {
     const int lane = r & 31;
     const long long row = (long long)t.row_base + t.m0 + r;
     const long long row0 = row - lane;
@@ -921,7 +921,7 @@ struct EpiDAct {
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
                                       bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
-                                      volatile int* abort_flag) const {
+                                      volatile int* abort_flag, int kernel_id) const {
     const int lane = r & 31;
     const long long row = (long long)t.row_base + t.m0 + r;
     const long long row0 = row - lane;
@@ -948,7 +948,7 @@ struct EpiDAct {
         }
         __syncwarp();
         if (!mbar_wait(wbar + (k & 1), (k >> 1) & 1, a.timeout_ns, abort_flag)) {
-          if (lane == 0) report_status(a.status, kStatusMbarTimeout, kKernelIdGemm2, 510 + k, 0, 0);
+          if (lane == 0) report_status(a.status, kStatusMbarTimeout, kernel_id, 510 + k, 0, 0);
           return;
         }
 #pragma unroll
@@ -1076,7 +1076,7 @@ struct EpiScatter {
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
                                       bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
-                                      volatile int* abort_flag) const {
+                                      volatile int* abort_flag, int kernel_id) const {
     const int lane = r & 31;
     const long long row = (long long)t.row_base + t.m0 + r;
     const bool row_ok = r < t.rows_valid;
@@ -1139,7 +1139,7 @@ struct EpiColScatter {
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
                                       bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
-                                      volatile int* abort_flag) const {
+                                      volatile int* abort_flag, int kernel_id) const {
     const int lane = r & 31;
     const long long row0 = (long long)t.row_base + t.m0 + (r - lane);
     const bool row_ok = r < t.rows_valid;

@@ -542,7 +542,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       epi.template run<BN>(t, args, taddr, q * 32 + lane, t.nk == 0, chalf,
-                           stg, maps.m, wbar, abort_flag);
+                           stg, maps.m, wbar, abort_flag, kKernelIdGemm);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[acc]);
@@ -843,7 +843,7 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       epi.template run<BN>(mine, args, taddr, q * 32 + lane, t.nk == 0, chalf,
-                           stg, maps.m, wbar, abort_flag);
+                           stg, maps.m, wbar, abort_flag, kKernelIdGemm2);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {
