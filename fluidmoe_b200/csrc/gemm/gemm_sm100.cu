@@ -275,6 +275,17 @@ struct BoxStore {
   }
 };
 
+// Phase of the barrier of block k's set in the epilogues that update whole blocks in place, two sets of boxes in
+// turn.  With four blocks a tile (BN 256) each set is filled twice, so every tile starts at phase 0; with two (BN 128)
+// once, so the phase turns with the tiles that the warp has done this way (`fills`).
+// Tiles of 128 columns by boxes against the path through registers: GELU gradient of 32768 rows, 64 -> 128 columns, 32.7 ->
+// 19.6 us, 2048 -> 128 57 -> 43; AdamW of 14336 x 128, 4096 rows, 42 -> 36.
+template <int kBlocks>
+__device__ __forceinline__ uint32_t box_parity(int k, uint32_t fills) {
+  static_assert(kBlocks == 2 || kBlocks == 4, "tiles of 128 or 256 columns");
+  return kBlocks == 4 ? (k >> 1) & 1 : fills & 1;
+}
+
 // ----------------------------------------------------------------------------------------
 // Epilogue 0: plain store (bf16 or fp32, optional accumulate; the fp32-accumulate form is the
 // weight-gradient epilogue that adds straight into a flat gradient buffer).
@@ -294,7 +305,7 @@ struct EpiStore {
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
                                       bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
-                                      volatile int* abort_flag, int kernel_id) const {
+                                      volatile int* abort_flag, int kernel_id, uint32_t& fills) const {
     const int lane = r & 31;
     const long long row = a.mode == 0 ? (long long)t.row_base + t.m0 + r : (long long)t.m0 + r;
     const long long row0 = row - lane;   // first row of this warp
@@ -527,8 +538,7 @@ struct EpiAdam {
   static constexpr int kWarpBytes = 2 * 3 * kBox;
   template <int BN>
   __device__ __forceinline__ bool whole(const Tile& t, const GemmArgs& a, int r, int chalf) const {
-    // four blocks a tile (BN 256): each set is filled twice, so its barrier's phase starts every tile at 0
-    return BN == 256 && boxes && t.rows_valid - (r & ~31) >= 32 && t.n_tile * BN + (chalf + 1) * (BN / 2) <= a.N;
+    return boxes && t.rows_valid - (r & ~31) >= 32 && t.n_tile * BN + (chalf + 1) * (BN / 2) <= a.N;
   }
   __device__ __forceinline__ void load_set(const CUtensorMap* maps, uint8_t* set, uint64_t* bar, int col, int row,
                                            int g) const {
@@ -578,7 +588,7 @@ struct EpiAdam {
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
                                       bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
-                                      volatile int* abort_flag, int kernel_id) const {
+                                      volatile int* abort_flag, int kernel_id, uint32_t& fills) const {
     constexpr int NB = BN / 64;          // 32-column blocks handled by this warp
     const int lane = r & 31;
     const long long row = a.mode == 0 ? (long long)t.row_base + t.m0 + r : (long long)t.m0 + r;
@@ -605,7 +615,7 @@ struct EpiAdam {
           load_set(maps, sets + ((k + 1) & 1) * 3 * kBox, wbar + ((k + 1) & 1), col + 32, (int)row0, z);
         }
         __syncwarp();
-        if (!mbar_wait(wbar + (k & 1), (k >> 1) & 1, a.timeout_ns, abort_flag)) {
+        if (!mbar_wait(wbar + (k & 1), box_parity<BN / 64>(k, fills), a.timeout_ns, abort_flag)) {
           if (lane == 0) report_status(a.status, kStatusMbarTimeout, kernel_id, 500 + k, 0, 0);
           return;
         }
@@ -627,6 +637,7 @@ struct EpiAdam {
         }
       }
       __syncwarp();
+      ++fills;
       return;
     }
     if (boxes) {
@@ -746,7 +757,7 @@ struct EpiAct {
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
                                       bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
-                                      volatile int* abort_flag, int kernel_id) const {
+                                      volatile int* abort_flag, int kernel_id, uint32_t& fills) const {
     const int lane = r & 31;
     const long long row = (long long)t.row_base + t.m0 + r;
     const long long row0 = row - lane;
@@ -877,8 +888,7 @@ struct EpiDAct {
   static constexpr int kWarpBytes = 2 * 2 * kBox;
   template <int BN>
   __device__ __forceinline__ bool whole(const Tile& t, const GemmArgs& a, int r, int chalf) const {
-    // four blocks a tile (BN 256): each set is filled twice, so its barrier's phase starts every tile at 0
-    return BN == 256 && boxes && t.rows_valid - (r & ~31) >= 32 && t.n_tile * BN + (chalf + 1) * (BN / 2) <= a.N;
+    return boxes && t.rows_valid - (r & ~31) >= 32 && t.n_tile * BN + (chalf + 1) * (BN / 2) <= a.N;
   }
   __device__ __forceinline__ void load_set(const CUtensorMap* maps, uint8_t* set, uint64_t* bar, int col,
                                            int row) const {
@@ -921,7 +931,7 @@ struct EpiDAct {
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
                                       bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
-                                      volatile int* abort_flag, int kernel_id) const {
+                                      volatile int* abort_flag, int kernel_id, uint32_t& fills) const {
     const int lane = r & 31;
     const long long row = (long long)t.row_base + t.m0 + r;
     const long long row0 = row - lane;
@@ -947,7 +957,7 @@ struct EpiDAct {
           load_set(maps, sets + ((k + 1) & 1) * 2 * kBox, wbar + ((k + 1) & 1), col + 32, (int)row0);
         }
         __syncwarp();
-        if (!mbar_wait(wbar + (k & 1), (k >> 1) & 1, a.timeout_ns, abort_flag)) {
+        if (!mbar_wait(wbar + (k & 1), box_parity<BN / 64>(k, fills), a.timeout_ns, abort_flag)) {
           if (lane == 0) report_status(a.status, kStatusMbarTimeout, kernel_id, 510 + k, 0, 0);
           return;
         }
@@ -1003,6 +1013,7 @@ struct EpiDAct {
         }
       }
       __syncwarp();
+      ++fills;
       dp = (d4[0] + d4[1]) + (d4[2] + d4[3]);
       if (dprobs_partial) dprobs_partial[(row * n_tiles + t.n_tile) * 2 + chalf] = dp;
       return;
@@ -1076,7 +1087,7 @@ struct EpiScatter {
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
                                       bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
-                                      volatile int* abort_flag, int kernel_id) const {
+                                      volatile int* abort_flag, int kernel_id, uint32_t& fills) const {
     const int lane = r & 31;
     const long long row = (long long)t.row_base + t.m0 + r;
     const bool row_ok = r < t.rows_valid;
@@ -1139,7 +1150,7 @@ struct EpiColScatter {
   template <int BN>
   __device__ __forceinline__ void run(const Tile& t, const GemmArgs& a, uint32_t taddr, int r,
                                       bool zero, int chalf, float* stg, const CUtensorMap* maps, uint64_t* wbar,
-                                      volatile int* abort_flag, int kernel_id) const {
+                                      volatile int* abort_flag, int kernel_id, uint32_t& fills) const {
     const int lane = r & 31;
     const long long row0 = (long long)t.row_base + t.m0 + (r - lane);
     const bool row_ok = r < t.rows_valid;

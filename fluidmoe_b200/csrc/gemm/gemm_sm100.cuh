@@ -292,7 +292,7 @@ struct GateKSource {
 
 template <int BN, class Epi>
 constexpr int gemm_stages() {
-  return (BN == 256 ? 3 : 4) - (EpiStaging<Epi>::bytes > 4 * kEpiStageFloats ? 1 : 0);
+  return BN == 128 ? 4 : EpiStaging<Epi>::bytes > 4 * kEpiStageFloats ? 2 : 3;
 }
 template <int BN, class Epi>
 constexpr int gemm_smem_bytes() {
@@ -522,6 +522,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
     const int chalf = (warp - 2) >> 2;  // which half of the tile's columns this warp drains
     float* stg = epi_stage + (warp - 2) * (EpiStaging<Epi>::bytes / 4);
     uint64_t* wbar = bars + kWarpBarOffset / 8 + 2 * (warp - 2);
+    uint32_t fills = 0;                 // tiles that the epilogue has updated in this warp's boxes
     TileWalker<BN> walker(args);
     TileWalker<BN> peek(args);
     Tile t;
@@ -542,7 +543,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       epi.template run<BN>(t, args, taddr, q * 32 + lane, t.nk == 0, chalf,
-                           stg, maps.m, wbar, abort_flag, kKernelIdGemm);
+                           stg, maps.m, wbar, abort_flag, kKernelIdGemm, fills);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[acc]);
@@ -805,6 +806,7 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
     const int chalf = (warp - 2) >> 2;
     float* stg = epi_stage + (warp - 2) * (EpiStaging<Epi>::bytes / 4);
     uint64_t* wbar = bars + kWarpBarOffset / 8 + 2 * (warp - 2);
+    uint32_t fills = 0;                 // tiles that the epilogue has updated in this warp's boxes
     TileWalker<BN, 2 * kBM> walker(args);
     TileWalker<BN, 2 * kBM> peek(args);
     const TileOrder order(args, pair_id, num_pairs);
@@ -843,7 +845,7 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       epi.template run<BN>(mine, args, taddr, q * 32 + lane, t.nk == 0, chalf,
-                           stg, maps.m, wbar, abort_flag, kKernelIdGemm2);
+                           stg, maps.m, wbar, abort_flag, kKernelIdGemm2, fills);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {

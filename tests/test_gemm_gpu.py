@@ -448,3 +448,63 @@ def test_residual_store_with_a_cut_last_block(N, in_place, cta_pair, monkeypatch
         assert torch.equal(out, first)
     torch.cuda.synchronize()
     gemm.check_status()
+
+
+@pytest.mark.parametrize("F", [128, 104, 64, 40])
+@pytest.mark.parametrize("act", ["gelu", "silu", "none"])
+def test_activation_gradient_of_narrow_tiles(F, act):
+    """Tiles of 128 columns, three a CTA: the boxes' barriers change phase with every tile.  Blocks that reach past F
+    (104: those of the second half of the columns) and groups' ends go through registers."""
+    torch.manual_seed(F)
+    rows = [30_000, 33, 0, 20_015]
+    G, H, total = len(rows), 64, sum(rows)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
+    offs = [sum(rows[:g]) for g in range(G)]
+    w2, dy, pre, probs = _rand(G, F, H, scale=0.1), _rand(total, H), _rand(total, F), torch.rand(total, device="cuda")
+    results = []
+    for lead in (0, 1):      # bases off 16 bytes go through registers
+        dpre = torch.full((total * F + 8,), 7.0, dtype=torch.bfloat16, device="cuda")[lead:lead + total * F].view(total, F)
+        src = torch.empty(total * F + 8, dtype=torch.bfloat16, device="cuda")[lead:lead + total * F].view(total, F)
+        src.copy_(pre)
+        results.append(gemm.grouped_gemm_dact(dy, w2, src, probs, activation=act, group_rows=i32(rows),
+                                              group_offs=i32(offs), dpre_out=dpre))
+    torch.cuda.synchronize()
+    gemm.check_status()
+    for g in range(G):
+        r = slice(offs[g], offs[g] + rows[g])
+        if rows[g] == 0:
+            continue
+        z = pre[r].double().requires_grad_(True)
+        y = gemm.act_ref(z, act)
+        d = dy[r].double() @ w2[g].double().t()
+        ref = torch.autograd.grad(y, z, d * probs[r].double()[:, None])[0]
+        dp = (d * y.detach()).sum(1)
+        for dpre, dprobs in results:
+            # one rounding of bf16 (2^-8) after fp32 sums and fast exponentials
+            assert ((dpre[r].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-4 * ref.abs().max()).all()
+            assert ((dprobs[r].double() - dp).abs() <= 1e-5 * dp.abs() + 2e-4 * dp.abs().max()).all()
+
+
+@pytest.mark.parametrize("N", [128, 104, 64])
+def test_wgrad_adam_of_narrow_tiles(N):
+    """Tiles of 128 columns, three a CTA: see above.  From the same start both paths agree to one rounding of bf16 (2^-7
+    between neighbours); before it they differ by a few 2^-23 of terms below 8, which is what is left where a weight
+    and its update cancel."""
+    torch.manual_seed(N)
+    G, rows, M = 2, 128, 30_000
+    x, dy = _rand(G * rows, M), _rand(G * rows, N)
+    start = [_rand(G, M, N), _rand(G, M, N, scale=0.1), _rand(G, M, N, scale=0.1).abs()]
+    results = []
+    for lead in (0, 1):
+        arrays = [torch.empty(G * M * N + 8, dtype=torch.bfloat16, device="cuda")[lead:lead + G * M * N].view(G, M, N)
+                  for _ in start]
+        for a, s in zip(arrays, start):
+            a.copy_(s)
+        gemm.grouped_gemm_wgrad_adam(x, dy, G, *arrays, lr=1e-2, beta1=0.9, beta2=0.99, eps=1e-8,
+                                     weight_decay=0.1, step=1, uniform_rows=rows, grad_scale=0.5)
+        results.append(arrays)
+    torch.cuda.synchronize()
+    gemm.check_status()
+    for s, box, reg in zip(start, *results):
+        assert not torch.equal(s, box)
+        torch.testing.assert_close(box.float(), reg.float(), rtol=2.0 ** -7, atol=4 * 8 * 2.0 ** -23)
