@@ -149,8 +149,8 @@ def grouped_gemm(
         holes = group_rows is not None and (zero_fill or not _native.use_native(a, b))
         out = (torch.zeros if holes else torch.empty)(a.shape[0], N, dtype=out_dtype, device=a.device)
     if residual is not None:
-        assert not accumulate and residual.shape == out.shape and residual.dtype == out.dtype == torch.bfloat16 \
-            and residual.stride(1) == 1 or not a.is_cuda
+        assert not accumulate and residual.shape == out.shape and residual.dtype == out.dtype
+        assert not a.is_cuda or (out.dtype == torch.bfloat16 and residual.stride(1) == 1)
     if not _native.use_native(a, b):
         if alpha_dev is not None:
             alpha = alpha * float(alpha_dev)
