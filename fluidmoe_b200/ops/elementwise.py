@@ -61,17 +61,18 @@ _ROPE_TABLES = {}
 
 
 def _cos_sin_table(freqs, rot):
-    """``[positions, rot, 2]`` fp32 (cos, sin) of the angle tensor, computed once per angle tensor
-    (keyed by storage address, shape and in-place version; a few entries are kept)."""
-    key = (freqs.data_ptr(), tuple(freqs.shape), freqs._version, str(freqs.device))
-    tab = _ROPE_TABLES.get(key)
-    if tab is None:
+    """``[positions, rot, 2]`` fp32 (cos, sin) of the angle tensor, computed once per angle tensor (keyed by
+    storage address, shape, strides and in-place version; a few entries are kept).  An entry keeps its angle tensor
+    too: as long as it is there no other tensor can have come to that address."""
+    key = (freqs.data_ptr(), tuple(freqs.shape), freqs.stride(), freqs.dtype, freqs._version, str(freqs.device))
+    entry = _ROPE_TABLES.get(key)
+    if entry is None:
         f = freqs.reshape(-1, rot).to(torch.float32)
-        tab = torch.stack((torch.cos(f), torch.sin(f)), dim=-1).contiguous()
+        entry = (torch.stack((torch.cos(f), torch.sin(f)), dim=-1).contiguous(), freqs)
         if len(_ROPE_TABLES) >= 8:
             _ROPE_TABLES.pop(next(iter(_ROPE_TABLES)))
-        _ROPE_TABLES[key] = tab
-    return tab
+        _ROPE_TABLES[key] = entry
+    return entry[0]
 
 
 def rope_packed_(qkv, freqs, q_per_group, head_dim, backward, wait=None):
