@@ -1264,7 +1264,7 @@ struct FlashBwdArgs {
 
 constexpr int kKernelIdDeltaWait = 17;
 __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
-                                  float* __restrict__ delta, int s, int b, int hq, const int* wait_flags,
+                                  bool out_by_8, float* __restrict__ delta, int s, int b, int hq, const int* wait_flags,
                                   int wait_n, int wait_expected, unsigned long long* wait_ns,
                                   unsigned long long timeout_ns, int* status) {
   // first consumer of the output gradient that peers fill (SP -> HP exchange of the backward pass)
@@ -1283,7 +1283,13 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const _
     const long long w = w0 + 2 * u;
     o[u] = g[u] = make_uint4(0, 0, 0, 0);
     if (w < total) {
-      o[u] = reinterpret_cast<const uint4*>(out + w * kFaD)[sub];
+      const __nv_bfloat16* op = out + w * kFaD + sub * 8;
+      if (out_by_8) {      // dout is a tensor map's base and always 16-byte aligned, the output need not be
+        const uint2 lo = reinterpret_cast<const uint2*>(op)[0], hi = reinterpret_cast<const uint2*>(op)[1];
+        o[u] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+      } else {
+        o[u] = *reinterpret_cast<const uint4*>(op);
+      }
       g[u] = reinterpret_cast<const uint4*>(dout + w * kFaD)[sub];
     }
   }
@@ -2332,6 +2338,10 @@ extern "C" int fm_flash_attn_bwd_gated(const void* qkv, const void* out, const v
     fm_set_error("flash_attn_bwd: buffers must be 16-byte aligned");
     return -1;
   }
+  if (reinterpret_cast<uintptr_t>(out) & 7) {
+    fm_set_error("flash_attn_bwd: the output must be 8-byte aligned");
+    return -1;
+  }
   CUtensorMap tq, tdo;
   if (!make_rows_tmap(&tq, qkv, (long long)b * G * (qpg + 2) * d, s) ||
       !make_rows_tmap(&tdo, dout, (long long)b * hq * d, s)) {
@@ -2340,7 +2350,8 @@ extern "C" int fm_flash_attn_bwd_gated(const void* qkv, const void* out, const v
   }
   const long long nrows = (long long)s * b * hq;
   fm::attn_delta_kernel<<<(unsigned)((nrows + 63) / 64), 256, 0, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(out), reinterpret_cast<const __nv_bfloat16*>(dout), delta, s, b, hq,
+      reinterpret_cast<const __nv_bfloat16*>(out), reinterpret_cast<const __nv_bfloat16*>(dout),
+      (reinterpret_cast<uintptr_t>(out) & 15) != 0, delta, s, b, hq,
       wait_flags, wait_n, wait_expected, wait_ns, timeout_ns ? timeout_ns : 4000000000ull, status);
   constexpr int smem = 6 * fm::kTileBytes + 1024 + 256;
   static bool configured = false;

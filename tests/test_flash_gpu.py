@@ -116,3 +116,28 @@ def test_flash_bwd_speed(version):
     ms = st.elapsed_time(en) / 5
     flops = 2.5 * 4 * s * s * G * qpg * d / 2
     print(f"\nflash bwd v{version} s={s} heads={G*qpg}: {ms:.3f} ms, {flops / ms / 1e9:.1f} TFLOP/s")
+
+
+@pytest.mark.parametrize("lead", [0, 4, 1])
+@pytest.mark.parametrize("s,b,G,qpg", [(1, 1, 1, 1), (130, 2, 1, 3)])
+def test_attention_backward_takes_an_output_off_16_bytes(lead, s, b, G, qpg):
+    """The saved output may lie on 8 bytes (the products of the row sums are read in halves then); anything less is
+    refused."""
+    d = 128
+    torch.manual_seed(s)
+    qkv = torch.randn(s, b, G, (qpg + 2) * d, device="cuda").bfloat16()
+    scale = 1.0 / math.sqrt(d)
+    out, lse = flash.flash_attn_fwd_packed(qkv, qpg, d, scale)
+    dout = torch.randn_like(out)
+    moved = torch.empty(out.numel() + 8, dtype=out.dtype, device="cuda")[lead:lead + out.numel()].view_as(out)
+    moved.copy_(out)
+    if lead == 1:
+        with pytest.raises(RuntimeError, match="8-byte aligned"):
+            flash.flash_attn_bwd_packed(dout, qkv, moved, lse, qpg, d, scale)
+        return
+    got = flash.flash_attn_bwd_packed(dout, qkv, moved, lse, qpg, d, scale)
+    ref = flash.flash_attn_bwd_packed(dout, qkv, out, lse, qpg, d, scale)
+    torch.cuda.synchronize()
+    gemm.check_status()
+    # the same row sums; dq is added up by atomics in fp32 before its one rounding
+    torch.testing.assert_close(got.float(), ref.float(), rtol=2.0 ** -7, atol=1e-5)
