@@ -285,3 +285,16 @@ def test_waiting_unpermute_gives_the_same(T, k):
                 status=gemm.status_buffer(rows.device).data_ptr())
     assert torch.equal(elementwise.unpermute_reduce(rows, slot, res, wait), elementwise.unpermute_reduce(rows, slot, res))
     gemm.check_status()
+
+
+@pytest.mark.parametrize("T,H,E,own", [(64, 512, 8, True), (4095, 2048, 64, True), (4096, 2048, 64, False), (4096, 4096, 8, False)])
+def test_router_input_gradient_of_many_rows_goes_to_the_library(T, H, E, own):
+    from fluidmoe_b200.ops import gemm, router
+    torch.manual_seed(T)
+    dl, w = torch.randn(T, E, device="cuda"), _rand(H, E)
+    before = gemm.LAUNCHES
+    got = router.router_dgrad(dl, w, torch.bfloat16)
+    assert (gemm.LAUNCHES > before) == own
+    ref = dl.bfloat16().double() @ w.double().t()
+    # fp32 sums of E products, then one rounding of bf16
+    assert ((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * E ** 0.5).all()
