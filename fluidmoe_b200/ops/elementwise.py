@@ -8,6 +8,7 @@ from typing import Optional
 import torch
 
 from .. import _native
+from .gemm import status_buffer
 
 LAUNCHES = 0
 
@@ -232,7 +233,6 @@ def embedding_grad_(main, ids, dy) -> bool:
     dy, ids = dy.contiguous(), ids.contiguous()
     if dy.data_ptr() % 16:
         return False
-    from .gemm import status_buffer
     _native.lib().embedding_grad(ids.data_ptr(), dy.data_ptr(), main.data_ptr(), dy.shape[0], dy.shape[1],
                                  main.shape[0], status_buffer(main.device).data_ptr(), _s())
     return True
