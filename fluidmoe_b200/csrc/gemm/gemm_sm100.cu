@@ -465,10 +465,10 @@ __device__ __forceinline__ void get_block_bf16(float* stg, int lane, float* v, i
 // (12 bytes of traffic per element instead of a 4-byte gradient store here plus a 16-byte
 // optimizer pass later).  Only valid when the gradient is complete after this GEMM: a single
 // micro-batch per step and no data-parallel reduction of this parameter.
-// Bound by memory now (12 bytes an element: 1.7 ms for 8 x 4096 x 28672).  With loads and stores from registers
-// the eight epilogue warps spent their time on the way to L2 (requests 56 % busy, a third of the stalls
-// `lg_throttle`) and on a trip of the accumulator through shared memory; through boxes, with one pipeline
-// stage less, 8 experts of 1024 rows take 3.70 -> 2.69 ms for 4096 x 28672 and 1.78 -> 1.32 ms for
+// 12 bytes an element, which the copy rate would move in 1.7 ms for 8 x 4096 x 28672; it takes 2.69 (4.2 TB/s).  With
+// loads and stores from registers the eight epilogue warps spent their time on the way to L2 (requests 56 % busy,
+// a third of the stalls `lg_throttle`) and on a trip of the accumulator through shared memory; through boxes, with
+// one pipeline stage less, 8 experts of 1024 rows take 3.70 -> 2.69 ms for 4096 x 28672 and 1.78 -> 1.32 ms for
 // 14336 x 4096.
 // ----------------------------------------------------------------------------------------
 struct EpiAdam {
@@ -493,9 +493,8 @@ struct EpiAdam {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
   }
-  // The arithmetic runs on packed fp32 pairs (fma.rn.f32x2 and friends, one issue slot per two
-  // elements): the eight epilogue warps are bound by instruction issue and dependency latency, not
-  // by the memory system, so halving the fp32 instruction count is what shortens the epilogue.
+  // The arithmetic runs on packed fp32 pairs (fma.rn.f32x2 and friends, one issue slot per two elements): the eight
+  // epilogue warps hide little latency, so fewer instructions in their chains are what the arithmetic can give.
   __device__ __forceinline__ void update8(const float* gg, uint4& pw, uint4& pm, uint4& pv) const {
     uint32_t* ww = reinterpret_cast<uint32_t*>(&pw);
     uint32_t* wm = reinterpret_cast<uint32_t*>(&pm);
@@ -1269,7 +1268,8 @@ static bool make_tmap_mn3d(CUtensorMap* m, const void* ptr, long long inner, lon
 }
 
 // Tensor map of an epilogue output [groups][rows][cols] (row stride `ld`, group stride `gs` elements) with
-// boxes of 32 rows x 128 (or 64) bytes in the swizzle of that width.  False when the addresses or strides do not allow it (16-byte rule).
+// boxes of 32 rows x 128 (or 64) bytes in the swizzle of that width.  False when the addresses or strides do not
+// allow it (16-byte rule).
 static bool make_out_map(CUtensorMap* m, const void* ptr, bool fp32, long long cols, long long rows, long long ld,
                          long long groups, long long gs, int row_bytes = 128) {
   EncodeTiledFn enc = get_encode();
@@ -1288,7 +1288,8 @@ static bool make_out_map(CUtensorMap* m, const void* ptr, bool fp32, long long c
   cuuint32_t estr[3] = {1, 1, 1};
   return enc(m, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr),
              dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+             row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 static int sm_count() {

@@ -3,8 +3,9 @@
 // One CTA (or a CTA pair sharing a 256 x BN tile through tcgen05.mma.cta_group::2) per SM walks a
 // list of output tiles: a static one for the single CTA, one claimed tile by tile from a counter for
 // the CTA pair (`TileOrder`), so that pairs which start late, because a collective kernel holds
-// their SMs, do fewer tiles instead of making the whole GEMM late.  Warp 0 feeds a shared-memory ring (5 stages for the CTA pair, 4 or 3
-// for a single CTA) with TMA tiled loads
+// their SMs, do fewer tiles instead of making the whole GEMM late.  Warp 0 feeds a shared-memory ring with TMA
+// tiled loads: five stages for the CTA pair and three for a single CTA with 256 columns, one less with the
+// AdamW epilogue, whose boxes take that room; four with 128 columns
 // (128-byte swizzle), warp 1 issues tcgen05.mma with the accumulator in TMEM (two accumulators, so
 // the epilogue of tile i overlaps the main loop of tile i+1), warps 2-9 (two per TMEM lane quarter,
 // each half of the columns) drain TMEM with tcgen05.ld and run a pluggable epilogue.  A pluggable
@@ -28,7 +29,6 @@ namespace fm {
 
 constexpr int kBM = 128;
 constexpr int kBK = 64;
-constexpr int kStages = 4;                 // BN = 128; the 256-wide single-CTA tile uses 3
 // Staging area of an epilogue warp: two boxes of 32 rows x 128 bytes for bulk tensor stores, or one
 // 32 x 32 fp32 block with padded rows.
 constexpr int kEpiBoxBytes = 32 * 128;
@@ -574,9 +574,9 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
 // CTA-pair variant: two CTAs of a cluster compute one 256 x 256 tile with
 // tcgen05.mma.cta_group::2.  Each CTA loads its own 128 rows of A and its own 128 columns of
 // B (no multicast), so every MMA reads half the shared-memory bytes per CTA that the
-// single-CTA kernel reads, and five pipeline stages fit beside the epilogue staging area.  CTA 0 of the pair issues the MMAs;
-// completion is broadcast to both CTAs' barriers with tcgen05.commit (multicast of the
-// *arrival*, not of a load).  Each CTA drains its own 128 accumulator rows from its own TMEM.
+// single-CTA kernel reads, and five pipeline stages fit beside the epilogue staging area (four beside the boxes of
+// the AdamW epilogue).  CTA 0 of the pair issues the MMAs; completion is broadcast to both CTAs' barriers with
+// tcgen05.commit (multicast of the *arrival*, not of a load).  Each CTA drains its own 128 accumulator rows from its own TMEM.
 // =========================================================================================
 template <class Epi>
 constexpr int gemm2_stages() {

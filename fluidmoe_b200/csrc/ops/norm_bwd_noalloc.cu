@@ -1,7 +1,7 @@
 // Normalisation backward that allocates nothing: the partial weight / bias gradients live in a
 // scratch array that is part of the library image (see include/fm_noalloc.h for the contract
-// and for who needs this).  The arithmetic is the same as fm_norm_bwd in elementwise.cu; the
-// kernels are repeated here so that the regular path is left untouched.
+// and for who needs this).  The formulas are those of fm_norm_bwd in elementwise.cu, its sums run in another
+// order; the kernels are separate so that the regular path is left untouched.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -759,7 +759,8 @@ extern "C" int fm_dropless_plan_local(const long long* top_idx, const float* top
                                       long long* row_token, float* row_prob, int* slot_of_token,
                                       cudaStream_t s) {
   const long long n = (long long)T * k;
-  if (T < 1 || k < 1 || E < 1 || E > fm::kPlanThreads || n + 63ll * E > 2147483647ll - fm::kDropStep || rows_max < n + 63ll * E) {
+  if (T < 1 || k < 1 || E < 1 || E > fm::kPlanThreads || n + 63ll * E > 2147483647ll - fm::kDropStep ||
+      rows_max < n + 63ll * E) {
     fm_set_error("dropless_plan_local: at most 1024 experts, and room for every pair plus 63 rows per expert");
     return -1;
   }
