@@ -797,17 +797,26 @@ struct EpiAct {
           }
           bs.send(maps + 1, box, col, (int)row0, 0);
         } else {
-          uint8_t* box = bs.next<0>();
-          uint8_t* abox = bs.next<0>();
+          // The pre-activation is handed over before the activation is evaluated, so that one store is under way
+          // during the arithmetic; the block is fetched again for it.  GELU 4096 x 4096, K = 2048: 67.2 us with both
+          // boxes handed over together (64.2 through registers), 64.0 now; 128 x 512 12.6 (12.3), 11.6.
+          if (pre_out != nullptr) {
+            uint8_t* box = bs.next<1>();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              load_acc(taddr + (c + h) * 32, v, zero);
+              bs.put_bf16(box, h, v);
+            }
+            bs.send(maps, box, col, (int)row0, 0);
+          }
+          uint8_t* abox = bs.next<1>();
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             load_acc(taddr + (c + h) * 32, v, zero);
-            if (pre_out != nullptr) bs.put_bf16(box, h, v);
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = act_f(act_kind, v[i]) * p;
             bs.put_bf16(abox, h, v);
           }
-          if (pre_out != nullptr) bs.send(maps, box, col, (int)row0, 0);
           bs.send(maps + 1, abox, col, (int)row0, 0);
         }
       }
