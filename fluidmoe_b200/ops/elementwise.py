@@ -27,13 +27,13 @@ def _bf16(*ts) -> bool:
     return all(t is None or t.dtype == torch.bfloat16 for t in ts)
 
 
-_t_norm_fwd = _native.tensor_call("t_norm_fwd")
-_t_norm_bwd = _native.tensor_call("t_norm_bwd")
-_t_gather_rows = _native.tensor_call("t_gather_rows")
-_t_unpermute_reduce = _native.tensor_call("t_unpermute_reduce")
-_t_topk_softmax = _native.tensor_call("t_topk_softmax")
-_t_moe_plan = _native.tensor_call("t_moe_plan")
-_t_rope_packed = _native.tensor_call("t_rope_packed")
+_t_norm_fwd = _native.tensor_call(globals(), "t_norm_fwd")
+_t_norm_bwd = _native.tensor_call(globals(), "t_norm_bwd")
+_t_gather_rows = _native.tensor_call(globals(), "t_gather_rows")
+_t_unpermute_reduce = _native.tensor_call(globals(), "t_unpermute_reduce")
+_t_topk_softmax = _native.tensor_call(globals(), "t_topk_softmax")
+_t_moe_plan = _native.tensor_call(globals(), "t_moe_plan")
+_t_rope_packed = _native.tensor_call(globals(), "t_rope_packed")
 
 
 def _counted(res):

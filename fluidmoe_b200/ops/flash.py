@@ -14,8 +14,8 @@ VERSION = int(os.environ.get("FLUIDMOE_FLASH_VERSION", "0"))
 BWD_VERSION = int(os.environ.get("FLUIDMOE_FLASH_BWD_VERSION", "2"))
 
 
-_t_flash_fwd = _native.tensor_call("t_flash_fwd")
-_t_flash_bwd = _native.tensor_call("t_flash_bwd")
+_t_flash_fwd = _native.tensor_call(globals(), "t_flash_fwd")
+_t_flash_bwd = _native.tensor_call(globals(), "t_flash_bwd")
 
 
 def supported(qkv: torch.Tensor, head_dim: int) -> bool:

@@ -33,10 +33,10 @@ def status_ptr(t: torch.Tensor) -> int:
     return at if at is not None else status_buffer(t.device).data_ptr()
 
 
-_t_gemm = _native.tensor_call("t_gemm")
-_t_gemm_act = _native.tensor_call("t_gemm_act")
-_t_gemm_dact = _native.tensor_call("t_gemm_dact")
-_t_gemm_wgrad = _native.tensor_call("t_gemm_wgrad")
+_t_gemm = _native.tensor_call(globals(), "t_gemm")
+_t_gemm_act = _native.tensor_call(globals(), "t_gemm_act")
+_t_gemm_dact = _native.tensor_call(globals(), "t_gemm_dact")
+_t_gemm_wgrad = _native.tensor_call(globals(), "t_gemm_wgrad")
 _FP32_OUT = {None: -1, torch.float32: 1, torch.bfloat16: 0}
 _ACT = {"gelu": 0, "silu": 1, "swiglu": 1, "none": 2}       # FmAct
 
