@@ -287,6 +287,13 @@ struct GateKSource {
   }
 };
 
+// Which lane of a producer warp issues the loads: any one, or behind a gate lane 0, which waits in it.
+template <bool kGated>
+__device__ __forceinline__ bool producer_issues(int lane) {
+  if constexpr (kGated) return lane == 0;
+  else return elect_one();
+}
+
 // Pipeline stages that fit beside the epilogue's staging area.
 constexpr int kSmemMax = 227 * 1024;
 template <class Epi>
@@ -358,7 +365,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
 
   if (warp == 0) {
     // ------------------------------- TMA producer -------------------------------
-    // The warp walks the loop as a whole and one elected lane issues (see the CTA-pair kernel).
+    // The warp walks the loop as a whole and one lane issues (see the CTA-pair kernel).
     constexpr bool kGated = !std::is_same<Gate, GateNone>::value;
     TileWalker<BN> walker(args);
     Tile t;
@@ -384,7 +391,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
           ok = false;
           break;
         }
-        if (elect_one()) {
+        if (producer_issues<kGated>(lane)) {
           uint8_t* sa = smem + stage * STAGE_BYTES;
           uint8_t* sb = sa + A_BYTES;
           mbar_expect_tx(&full[stage], STAGE_BYTES);
@@ -654,6 +661,8 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
     // coordinate per block took 450 to 700 (its scheduler also serves two busy epilogue warps), so that short
     // contractions ran at the producer's pace, not at the tensor core's: 64 x 768 rows, 2048 x 2816 weight gradient 558 ->
     // 519 us, 64 x 1024 rows, 1024 -> 2048 232 -> 218, 3351 x 6144 x 2048 79 -> 75.
+    // Behind a gate that lane is lane 0, which has acquired the arrival counter: what peers stored is ordered before the
+    // loads of the lane that acquired, and a vote hands that order to no other.
     constexpr bool kGated = !std::is_same<Gate, GateNone>::value;
     TileWalker<BN, 2 * kBM> walker(args);
     const TileOrder order(args, pair_id, num_pairs);
@@ -712,7 +721,7 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tma_a,
           ok = false;
           break;
         }
-        if (elect_one()) {
+        if (producer_issues<kGated>(lane)) {
           uint8_t* sa = smem + stage * STAGE_BYTES;
           uint8_t* sb = sa + A_BYTES;
           if (leader) mbar_expect_tx(&full[stage], 2 * STAGE_BYTES);

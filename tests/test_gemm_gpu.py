@@ -508,3 +508,28 @@ def test_wgrad_adam_of_narrow_tiles(N):
     for s, box, reg in zip(start, *results):
         assert not torch.equal(s, box)
         torch.testing.assert_close(box.float(), reg.float(), rtol=2.0 ** -7, atol=4 * 8 * 2.0 ** -23)
+
+
+@pytest.mark.parametrize("cta_pair", [0, 1])
+@pytest.mark.parametrize("rows,N,expected", [(200, 264, 1), (333, 128, 3), (129, 520, 2)])
+def test_gated_rows_and_gated_columns_that_have_arrived(rows, N, expected, cta_pair, monkeypatch):
+    """The producers behind a gate, on counters that stand at their targets: blocks of 128 rows of a group, and
+    column blocks by their source, begun at another source than the first."""
+    monkeypatch.setattr(gemm, "CTA_PAIR", cta_pair)
+    torch.manual_seed(8)
+    G, K, per_src = 3, 256, 2
+    blocks = (rows + 127) // 128
+    a, w = _rand(G * rows, K), _rand(G, K, N)
+    in_block = torch.tensor([min(128, rows - 128 * i) for i in range(blocks)], dtype=torch.int32, device="cuda")
+    waited = torch.zeros(1, dtype=torch.int64, device="cuda")
+    common = dict(gate_blocks_per_group=blocks, gate_expected=expected, timeout_ns=10 ** 9, wait_ns=waited.data_ptr())
+    flags = (in_block * expected).repeat(G)
+    got = gemm.grouped_gemm(a, w, uniform_rows=rows, gate=dict(gate_flags=flags.data_ptr(), **common))
+    gemm.check_status()
+    for g in range(G):
+        _close(got[g * rows:(g + 1) * rows], a[g * rows:(g + 1) * rows].float() @ w[g].float())
+    flags = (in_block * expected).repeat(K // 64 // per_src)
+    got = gemm.grouped_gemm(a[:rows], w[:1], gate=dict(gate_flags=flags.data_ptr(), gate_k_blocks_per_src=per_src,
+                                                       k_rotate=per_src, **common))
+    gemm.check_status()
+    _close(got, a[:rows].float() @ w[0].float())
