@@ -50,7 +50,7 @@ constexpr bool few_act(int kind) { return kind >= kFewGelu; }
 
 struct FewArgs {
   int groups, N, nk, ntn;             // output columns, k blocks, tiles along N
-  int rows, total_rows;               // rows of every group but perhaps the last; rows of all
+  int rows, total_rows;               // rows of a group unless they end before; rows of all
   int w_group_stride;                 // rows of the flattened weights between groups
   int n_half;                         // columns between the two halves of a tile
   void* C;
@@ -558,7 +558,9 @@ int gemm_few_launch(const FmGemmDesc* d, cudaStream_t stream) {
   a.ntn = (d->N + tile_n - 1) / tile_n;
   // narrow products of one group: chunks of rows in the place of groups, all with the same weights
   a.rows = chunks ? kFewRows : d->uniform_rows;
-  a.total_rows = chunks ? d->uniform_rows : d->num_groups * d->uniform_rows;
+  // no more than A has: the last groups may be cut, or empty, as with the tiled GEMM's stores
+  const long long all_rows = (long long)(chunks ? 1 : d->num_groups) * d->uniform_rows;
+  a.total_rows = (int)(all_rows < d->a_outer ? all_rows : d->a_outer);
   a.w_group_stride = chunks ? 0 : d->b_group_stride;
   a.n_half = kind == kFewWide ? kFewCols : d->n_half;
   a.C = act ? d->act_out : d->C;

@@ -49,6 +49,27 @@ def test_store(monkeypatch, rows, groups, K, N, layout):
     gemm.check_status()
 
 
+@pytest.mark.parametrize("have,rows,N", [(40, 16, 4096), (17, 16, 264), (100, 60, 512), (16, 16, 4096)])
+def test_groups_beyond_the_rows(monkeypatch, have, rows, N):
+    """``uniform_rows`` of three groups may come to more rows than there are: the last groups are cut or empty, and
+    nothing behind the results is written."""
+    torch.manual_seed(5)
+    a, w, p = _r(have, 1024), _r(3, 1024, N), torch.rand(have, device="cuda")
+    want = torch.cat([a[g * rows:(g + 1) * rows].float() @ w[g].float() for g in range(3)])
+
+    def run(dtype):
+        room = torch.full((have + 2 * rows, N), 7.0, device="cuda", dtype=dtype)
+        gemm.grouped_gemm(a, w, uniform_rows=rows, out=room[:have])
+        assert (room[have:] == 7.0).all()
+        return room[:have]
+    for got in (run(torch.float32), _alone(monkeypatch, lambda: run(torch.float32))):
+        _close(got, want, 1e-5)
+    act, pre = gemm.grouped_gemm_act(a, w, p, activation="silu", uniform_rows=rows)
+    _close(act, gemm.act_ref(want, "silu") * p.unsqueeze(1), 4e-3)
+    _close(pre, want, 4e-3)
+    gemm.check_status()
+
+
 @pytest.mark.parametrize("rows", [33, 64, 100, 1000, 2016, 2017])
 @pytest.mark.parametrize("K,N,layout", [(2048, 8, "nk"), (2056, 72, "nk"), (2048, 128, "kn"), (4096, 64, "nk"),
                                         (2040, 64, "kn")])
