@@ -1356,12 +1356,13 @@ __global__ void attn_dq_store_kernel(const float* __restrict__ dq, __nv_bfloat16
 }
 
 // The same from the second-generation kernel's buffer: tiles of 128 query rows, [b, hq, tile], each as [32-row quarter][4
-// columns][row][4 values].  A CTA takes a tile; the lanes of a warp take eight rows x 32 columns at a time, so that
-// reads come in runs of 128 bytes and writes in runs of 64.
+// columns][row][4 values].  A CTA takes a tile (along one dimension of the grid: batches and heads may be more than 65535);
+// the lanes of a warp take eight rows x 32 columns at a time, so that reads come in runs of 128 bytes and writes in runs of 64.
 __global__ void attn_dq_store_tiled_kernel(const float* __restrict__ dq, __nv_bfloat16* __restrict__ dqkv, int s, int b,
                                            int G, int qpg, float mul) {
-  const int hq = G * qpg, h = blockIdx.y, bb = blockIdx.z, g = h / qpg, hi = h % qpg;
-  const float* tile = dq + ((long long)(bb * hq + h) * gridDim.x + blockIdx.x) * (kFaBM * kFaD);
+  const int nq = (s + kFaBM - 1) / kFaBM, bh = blockIdx.x / nq, i = blockIdx.x - bh * nq;
+  const int hq = G * qpg, bb = bh / hq, h = bh - bb * hq, g = h / qpg, hi = h - g * qpg;
+  const float* tile = dq + (long long)blockIdx.x * (kFaBM * kFaD);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r8 = lane & 7, c8 = lane >> 3;
 #pragma unroll
@@ -1372,7 +1373,7 @@ __global__ void attn_dq_store_tiled_kernel(const float* __restrict__ dq, __nv_bf
     uint4 p;
     p.x = pack_bf16x2(x.x * mul, x.y * mul); p.y = pack_bf16x2(x.z * mul, x.w * mul);
     p.z = pack_bf16x2(y.x * mul, y.y * mul); p.w = pack_bf16x2(y.z * mul, y.w * mul);
-    const long long pos = (long long)blockIdx.x * kFaBM + row;
+    const long long pos = (long long)i * kFaBM + row;
     if (pos < s) *reinterpret_cast<uint4*>(dqkv + (((pos * b + bb) * G + g) * (qpg + 2) + hi) * kFaD + col) = p;
   }
 }
@@ -2450,7 +2451,7 @@ extern "C" int fm_flash_attn_bwd_gated(const void* qkv, const void* out, const v
     }
     dim3 grid_lin(grid.x * grid.y * grid.z, 1, 1);
     fm::flash_bwd2_kernel<<<grid_lin, fm::kFaB2Threads, fm::kFaB2Smem, stream>>>(tq, tdo, a);
-    fm::attn_dq_store_tiled_kernel<<<dim3((s + 127) / 128, hq, b), 256, 0, stream>>>(dq_accum, a.dqkv, s, b, G, qpg, scale);
+    fm::attn_dq_store_tiled_kernel<<<(unsigned)((s + 127) / 128) * hq * b, 256, 0, stream>>>(dq_accum, a.dqkv, s, b, G, qpg, scale);
     if (a.hsplit > 1)
       fm::attn_dkv_store_kernel<<<148 * 4, 256, 0, stream>>>(dkv_accum, a.dqkv, (long long)s * b, G, qpg);
   } else {
