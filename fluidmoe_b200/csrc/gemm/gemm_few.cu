@@ -17,12 +17,11 @@
 #include <cuda_bf16.h>
 #include <string.h>
 
-#include <map>
 #include <mutex>
-#include <utility>
 
 #include "../include/fm_tmap.h"
 #include "../include/sm100_ptx.cuh"
+#include "../include/stream_table.h"
 #include "act_math.cuh"
 #include "gemm_few.h"
 
@@ -447,38 +446,28 @@ long long gemm_few_workspace(const FmGemmDesc* d) {
   return few_partial_bytes(d) + kFewCounters * (long long)sizeof(int);
 }
 
-// Counters of the shared tiles, one group of sets per (device, stream): launches on a stream run one after another and
-// use the sets in rotation; a launch clears the set that comes up half a rotation later.  Under capture, on the handle that
-// stands for another stream in each thread and beyond kFewStreams streams the counters lie in the workspace instead and a
-// node of their own clears them (2 us).
+// Counters of the shared tiles, one group of sets for a stream: launches on a stream run one after another and use the sets
+// in rotation; a launch clears the set that comes up half a rotation later.  Where the stream has none (under capture, and
+// beyond the streams that the table knows) the counters lie in the workspace and a node of their own clears them (2 us).
 class FewCounters {
  public:
   int *use = nullptr, *reset = nullptr;
   bool take(cudaStream_t stream, int* own) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return false;
-    }
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return false;
-    if (cap == cudaStreamCaptureStatusNone && stream != cudaStreamPerThread) {
-      std::lock_guard<std::mutex> lock(mu());
-      auto& table = sets();
-      const auto key = std::make_pair(dev, stream);
-      if (table.size() < kFewStreams || table.count(key)) {
-        Sets& s = table[key];
-        if (s.p == nullptr) s.p = fresh(stream);
-        if (s.p != nullptr) {
-          const unsigned i = s.next++ % kFewSets;
-          use = s.p + i * kFewCounters;
-          reset = s.p + (i + kFewSets / 2) % kFewSets * kFewCounters;
-          return true;
-        }
-      }
+    StreamTable<Sets>& t = table();
+    std::lock_guard<std::mutex> lock(t.mu);
+    Sets* s = nullptr;
+    if (!t.find(stream, &s)) return false;
+    if (s != nullptr && s->p == nullptr) s->p = fresh(stream);
+    if (s != nullptr && s->p != nullptr) {
+      const unsigned i = s->next++ % kFewSets;
+      use = s->p + i * kFewCounters;
+      reset = s->p + (i + kFewSets / 2) % kFewSets * kFewCounters;
+      return true;
     }
     use = own;
-    return cudaMemsetAsync(own, 0, kFewCounters * sizeof(int), stream) == cudaSuccess;
+    if (cudaMemsetAsync(own, 0, kFewCounters * sizeof(int), stream) == cudaSuccess) return true;
+    (void)cudaGetLastError();
+    return false;
   }
   // The launch that was to clear a set did not run.
   void unused(cudaStream_t stream) {
@@ -486,18 +475,13 @@ class FewCounters {
   }
 
  private:
-  static constexpr size_t kFewStreams = 64;
   struct Sets {
     int* p = nullptr;
     unsigned next = 0;
   };
-  static std::mutex& mu() {
-    static std::mutex m;
-    return m;
-  }
-  static std::map<std::pair<int, cudaStream_t>, Sets>& sets() {
-    static std::map<std::pair<int, cudaStream_t>, Sets> table;
-    return table;
+  static StreamTable<Sets>& table() {
+    static StreamTable<Sets> t;
+    return t;
   }
   static int* fresh(cudaStream_t stream) {
     const size_t bytes = (size_t)kFewSets * kFewCounters * sizeof(int);

@@ -4,12 +4,11 @@
 #include <stdlib.h>
 #include <string.h>
 
-#include <map>
 #include <mutex>
-#include <utility>
 
 #include "../include/fm_api.h"
 #include "../include/fm_tmap.h"
+#include "../include/stream_table.h"
 #include "act_math.cuh"
 #include "gemm_few.h"
 #include "gemm_sm100.cuh"
@@ -1249,11 +1248,11 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmAr
   return 0;
 }
 
-// Workspace of the dynamic tile order, one per (device, stream): launches on one stream run one
+// Workspace of the dynamic tile order, one for a stream: launches on one stream run one
 // after another, so they can share claim counters (used in rotation; a launch zeroes the counter
 // that comes up half a rotation later) and the log (entries carry the launch's epoch).  A stream
 // that is being captured into a graph keeps the static order, because a replay would repeat the
-// epoch of the capture.
+// epoch of the capture, and so do streams beyond those that the table knows.
 struct SchedWorkspace {
   int* ctrs = nullptr;
   unsigned long long* log = nullptr;
@@ -1280,17 +1279,11 @@ static void sched_prepare(GemmArgs& args, int pairs, long long tiles, cudaStream
   args.sched_cap = 0;
   args.sched_epoch = 0;
   if (!sched_dynamic_enabled() || tiles <= pairs || tiles > (1ll << 24)) return;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-    (void)cudaGetLastError();
-    return;
-  }
-  static std::mutex mu;
-  static std::map<std::pair<int, cudaStream_t>, SchedWorkspace> table;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lock(mu);
-  SchedWorkspace& ws = table[std::make_pair(dev, stream)];
+  static StreamTable<SchedWorkspace> table;
+  std::lock_guard<std::mutex> lock(table.mu);
+  SchedWorkspace* state = nullptr;
+  if (!table.find(stream, &state) || state == nullptr) return;
+  SchedWorkspace& ws = *state;
   if (ws.ctrs == nullptr) {
     if (cudaMalloc(&ws.ctrs, kSchedCounters * sizeof(int)) != cudaSuccess) {
       (void)cudaGetLastError();
