@@ -19,6 +19,7 @@
 
 #include <mutex>
 
+#include "../include/fm_smem.h"
 #include "../include/fm_tmap.h"
 #include "../include/sm100_ptx.cuh"
 #include "../include/stream_table.h"
@@ -501,17 +502,12 @@ template <int kKind, bool kMn, int NT>
 static int few_launch(const CUtensorMap& tw, const CUtensorMap& tx, const FewArgs& a, int grid, cudaStream_t stream) {
   auto kern = gemm_few_kernel<kKind, kMn, NT>;
   constexpr int smem = few_smem<kKind, NT>();
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) {
-      fm_set_error(cudaGetErrorString(e));
-      return (int)e;
-    }
-    configured = true;
+  static std::atomic<unsigned long long> configured{0};
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), smem, configured);
+  if (e == cudaSuccess) {
+    kern<<<grid, kFewThreads, smem, stream>>>(tw, tx, a);
+    e = cudaGetLastError();
   }
-  kern<<<grid, kFewThreads, smem, stream>>>(tw, tx, a);
-  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     fm_set_error(cudaGetErrorString(e));
     return (int)e;

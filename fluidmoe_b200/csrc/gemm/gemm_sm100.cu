@@ -7,6 +7,7 @@
 #include <mutex>
 
 #include "../include/fm_api.h"
+#include "../include/fm_smem.h"
 #include "../include/fm_tmap.h"
 #include "../include/stream_table.h"
 #include "act_math.cuh"
@@ -1230,17 +1231,14 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmAr
                       const Epi& epi, const Gate& gate, const OutMaps& maps, int grid, cudaStream_t stream) {
   auto kern = gemm_sm100_kernel<A_MN, B_MN, BN, Epi, Gate>;
   constexpr int smem = gemm_smem_bytes<BN, Epi>();
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) {
-      set_err(cudaGetErrorString(e));
-      return (int)e;
-    }
-    configured = true;
+  static std::atomic<unsigned long long> configured{0};
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), smem, configured);
+  if (e != cudaSuccess) {
+    set_err(cudaGetErrorString(e));
+    return (int)e;
   }
   kern<<<grid, kGemmThreads, smem, stream>>>(ta, tb, args, epi, gate, maps);
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_err(cudaGetErrorString(e));
     return (int)e;
@@ -1321,14 +1319,11 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
                        const Epi& epi, const Gate& gate, const OutMaps& maps, int grid, cudaStream_t stream) {
   auto kern = gemm2_sm100_kernel<A_MN, B_MN, Epi, Gate>;
   constexpr int smem = gemm2_smem_bytes<Epi>();
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) {
-      set_err(cudaGetErrorString(e));
-      return (int)e;
-    }
-    configured = true;
+  static std::atomic<unsigned long long> configured{0};
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), smem, configured);
+  if (e != cudaSuccess) {
+    set_err(cudaGetErrorString(e));
+    return (int)e;
   }
   // The kernel is persistent: never launch more pairs than can be resident at once (pairs must
   // sit on two SMs of one GPC, so this can be fewer than SMs / 2).
@@ -1358,7 +1353,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
   GemmArgs args = args_in;
   sched_prepare(args, grid / 2, args_in.sched_cap, stream);   // sched_cap arrives as the tile bound
   kern<<<grid, kGemmThreads, smem, stream>>>(ta, tb, args, epi, gate, maps);
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_err(cudaGetErrorString(e));
     return (int)e;

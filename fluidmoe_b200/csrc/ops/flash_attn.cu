@@ -23,6 +23,7 @@
 #include <stdio.h>
 
 #include "../include/fm_ops.h"
+#include "../include/fm_smem.h"
 #include "../include/fm_tmap.h"
 #include "../include/sm100_ptx.cuh"
 
@@ -2208,15 +2209,11 @@ extern "C" int fm_flash_attn_fwd_push(const void* qkv, void* out, float* lse, in
     return -3;
   }
   constexpr int smem = 6 * fm::kTileBytes + 1024 + 256;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(fm::flash_fwd_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) {
-      fm_set_error(cudaGetErrorString(e));
-      return (int)e;
-    }
-    configured = true;
+  static std::atomic<unsigned long long> configured{0};
+  cudaError_t e = fm::allow_smem(reinterpret_cast<const void*>(fm::flash_fwd_kernel), smem, configured);
+  if (e != cudaSuccess) {
+    fm_set_error(cudaGetErrorString(e));
+    return (int)e;
   }
   fm::FlashFwdArgs a;
   a.s = s; a.b = b; a.G = G; a.qpg = qpg;
@@ -2239,14 +2236,11 @@ extern "C" int fm_flash_attn_fwd_push(const void* qkv, void* out, float* lse, in
                                     fm::flash_fwd3_kernel<2>, fm::flash_fwd3_kernel<2>};
     const int variant = version == 3 ? fm::kFa3DefaultPoly : version - 30;
     constexpr int smem3 = (1 + 2 * fm::kFa3Stages) * fm::kTileBytes + 1024 + 2048;
-    static bool configured3[5] = {false, false, false, false, false};
-    if (!configured3[variant]) {
-      cudaError_t e3 = cudaFuncSetAttribute(kFwd3[variant], cudaFuncAttributeMaxDynamicSharedMemorySize, smem3);
-      if (e3 != cudaSuccess) {
-        fm_set_error(cudaGetErrorString(e3));
-        return (int)e3;
-      }
-      configured3[variant] = true;
+    static std::atomic<unsigned long long> configured3[5];
+    e = fm::allow_smem(reinterpret_cast<const void*>(kFwd3[variant]), smem3, configured3[variant]);
+    if (e != cudaSuccess) {
+      fm_set_error(cudaGetErrorString(e));
+      return (int)e;
     }
     const int nq3 = (s + fm::kFaBM - 1) / fm::kFaBM;
     dim3 grid3((unsigned)(nq3 * G * qpg * b), 1, 1);
@@ -2294,14 +2288,11 @@ extern "C" int fm_flash_attn_fwd_push(const void* qkv, void* out, float* lse, in
                                     fm::flash_fwd2_kernel<0, true, 4>};
     const int variant = version == 2 ? fm::kFa2DefaultPoly : version - 20;
     constexpr int smem2 = smem;
-    static bool configured2[9] = {false, false, false, false, false, false, false, false, false};
-    if (!configured2[variant]) {
-      cudaError_t e2 = cudaFuncSetAttribute(kFwd2[variant], cudaFuncAttributeMaxDynamicSharedMemorySize, smem2);
-      if (e2 != cudaSuccess) {
-        fm_set_error(cudaGetErrorString(e2));
-        return (int)e2;
-      }
-      configured2[variant] = true;
+    static std::atomic<unsigned long long> configured2[9];
+    e = fm::allow_smem(reinterpret_cast<const void*>(kFwd2[variant]), smem2, configured2[variant]);
+    if (e != cudaSuccess) {
+      fm_set_error(cudaGetErrorString(e));
+      return (int)e;
     }
     const int nq = (s + fm::kFaBM - 1) / fm::kFaBM;
     dim3 grid2((unsigned)(((nq + 1) / 2) * G * qpg * b), 1, 1);
@@ -2348,7 +2339,7 @@ extern "C" int fm_flash_attn_fwd_push(const void* qkv, void* out, float* lse, in
     dim3 grid((s + fm::kFaBM - 1) / fm::kFaBM, G * qpg, b);
     fm::flash_fwd_kernel<<<grid, fm::kFaThreads, smem, stream>>>(tmap, a);
   }
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) {
     fm_set_error(cudaGetErrorString(e));
     return (int)e;
@@ -2410,14 +2401,11 @@ extern "C" int fm_flash_attn_bwd_gated(const void* qkv, const void* out, const v
       (reinterpret_cast<uintptr_t>(out) & 15) != 0, delta, s, b, hq, reinterpret_cast<float4*>(dq_accum), dq_rows * hq * (d / 4),
       reinterpret_cast<float4*>(dkv_accum), dkv_accum != nullptr ? (long long)s * b * G * 2 * (d / 4) : 0, wait_flags, wait_n, wait_expected, wait_ns, timeout_ns ? timeout_ns : 4000000000ull, status);
   constexpr int smem = 6 * fm::kTileBytes + 1024 + 256;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(fm::flash_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) {
-      fm_set_error(cudaGetErrorString(e));
-      return (int)e;
-    }
-    configured = true;
+  static std::atomic<unsigned long long> configured{0};
+  cudaError_t e = fm::allow_smem(reinterpret_cast<const void*>(fm::flash_bwd_kernel), smem, configured);
+  if (e != cudaSuccess) {
+    fm_set_error(cudaGetErrorString(e));
+    return (int)e;
   }
   fm::FlashBwdArgs a;
   a.s = s; a.b = b; a.G = G; a.qpg = qpg;
@@ -2433,15 +2421,11 @@ extern "C" int fm_flash_attn_bwd_gated(const void* qkv, const void* out, const v
   a.dkv_accum = nullptr;
   dim3 grid((s + fm::kFaBN - 1) / fm::kFaBN, G, b);
   if (version == 2) {
-    static bool configured2 = false;
-    if (!configured2) {
-      cudaError_t e2 = cudaFuncSetAttribute(fm::flash_bwd2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            fm::kFaB2Smem);
-      if (e2 != cudaSuccess) {
-        fm_set_error(cudaGetErrorString(e2));
-        return (int)e2;
-      }
-      configured2 = true;
+    static std::atomic<unsigned long long> configured2{0};
+    e = fm::allow_smem(reinterpret_cast<const void*>(fm::flash_bwd2_kernel), fm::kFaB2Smem, configured2);
+    if (e != cudaSuccess) {
+      fm_set_error(cudaGetErrorString(e));
+      return (int)e;
     }
     if (hsplit > 1 && dkv_accum != nullptr && qpg % hsplit == 0 &&
         (reinterpret_cast<uintptr_t>(dkv_accum) & 15) == 0) {
@@ -2458,7 +2442,7 @@ extern "C" int fm_flash_attn_bwd_gated(const void* qkv, const void* out, const v
     fm::flash_bwd_kernel<<<grid, fm::kFaThreads, smem, stream>>>(tq, tdo, a);
     fm::attn_dq_store_kernel<<<148 * 8, 256, 0, stream>>>(dq_accum, a.dqkv, (long long)s * b, G, qpg, 1.0f);
   }
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) {
     fm_set_error(cudaGetErrorString(e));
     return (int)e;

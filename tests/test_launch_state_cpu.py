@@ -72,3 +72,30 @@ int main() {
   CHECK(t.find(handle, &b) && b == a && a->n == 7);
 }
 """)
+
+
+def test_shared_memory_limit_of_every_device(tmp_path):
+    """The limit is raised on each device that launches the kernel, once; a refusal is tried again."""
+    _run(tmp_path, CHECK + """
+#include "include/fm_smem.h"
+static int dev = 0, raised = 0;
+static cudaError_t answer = cudaSuccess;
+extern "C" cudaError_t cudaGetDevice(int* d) { *d = dev; return cudaSuccess; }
+extern "C" cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { ++raised; return answer; }
+int main() {
+  static std::atomic<unsigned long long> done{0}, other[2];
+  answer = cudaErrorInvalidValue;
+  CHECK(fm::allow_smem(&dev, 1, done) == cudaErrorInvalidValue && raised == 1);
+  answer = cudaSuccess;
+  for (int i = 0; i < 2; ++i) CHECK(fm::allow_smem(&dev, 1, done) == cudaSuccess && raised == 2);
+  dev = 1;
+  for (int i = 0; i < 2; ++i) CHECK(fm::allow_smem(&dev, 1, done) == cudaSuccess && raised == 3);
+  dev = 63;
+  for (int i = 0; i < 2; ++i) CHECK(fm::allow_smem(&dev, 1, done) == cudaSuccess && raised == 4);
+  dev = 64;
+  for (int i = 0; i < 2; ++i) CHECK(fm::allow_smem(&dev, 1, done) == cudaSuccess && raised == 5 + i);
+  dev = 0;
+  CHECK(fm::allow_smem(&dev, 1, done) == cudaSuccess && raised == 6);
+  CHECK(fm::allow_smem(&dev, 1, other[1]) == cudaSuccess && raised == 7);
+}
+""")
