@@ -30,7 +30,7 @@ static void check(int rc, const char* what) {
   if (rc != 0) throw std::runtime_error(std::string(what) + ": " + fm_last_error());
 }
 
-static void gemm_launch(const py::dict& d, uintptr_t stream) {
+static FmGemmDesc gemm_descriptor(const py::dict& d) {
   FmGemmDesc g{};
   g.A = reinterpret_cast<const void*>(field<uintptr_t>(d, FM_KEY("A"), 0));
   g.B = reinterpret_cast<const void*>(field<uintptr_t>(d, FM_KEY("B"), 0));
@@ -107,7 +107,15 @@ static void gemm_launch(const py::dict& d, uintptr_t stream) {
   g.timeout_ns = field<unsigned long long>(d, FM_KEY("timeout_ns"), 0ull);
   g.wait_ns = reinterpret_cast<unsigned long long*>(field<uintptr_t>(d, FM_KEY("wait_ns"), 0));
   g.status = reinterpret_cast<int*>(field<uintptr_t>(d, FM_KEY("status"), 0));
+  return g;
+}
+static void gemm_launch(const py::dict& d, uintptr_t stream) {
+  const FmGemmDesc g = gemm_descriptor(d);
   check(fm_gemm_launch(&g, reinterpret_cast<cudaStream_t>(stream)), "fm_gemm_launch");
+}
+static long long gemm_workspace(const py::dict& d) {
+  const FmGemmDesc g = gemm_descriptor(d);
+  return fm_gemm_workspace(&g);
 }
 
 void bind_ops(py::module_& m);   // ops_bindings.cpp
@@ -118,6 +126,7 @@ int fm_add_tensor_calls(PyObject* module);   // tensor_calls.cpp
 PYBIND11_MODULE(_C, m) {
   m.doc() = "fluidmoe_b200 native kernels (sm_100a)";
   m.def("gemm_launch", &gemm_launch, py::arg("desc"), py::arg("stream"));
+  m.def("gemm_workspace", &gemm_workspace, py::arg("desc"));
   m.def("last_error", []() { return std::string(fm_last_error()); });
   m.attr("EPI_STORE") = (int)FM_EPI_STORE;
   m.attr("EPI_ACT") = (int)FM_EPI_ACT;

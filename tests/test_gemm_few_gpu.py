@@ -6,6 +6,7 @@ probability): 4e-3 of the norm; fp32 results 1e-5."""
 import pytest
 import torch
 
+from fluidmoe_b200 import _native
 from fluidmoe_b200.ops import gemm
 
 pytestmark = pytest.mark.gpu
@@ -28,6 +29,29 @@ def _alone(monkeypatch, fn):
         return fn()
 
 
+def _taken(monkeypatch, fn):
+    """The call with scratch, which only the C++ call gives."""
+    made = []
+    with monkeypatch.context() as m:
+        for name in ("_t_gemm", "_t_gemm_act"):
+            def record(*args, call=getattr(gemm, name)):
+                made.append(call(*args))
+                return made[-1]
+            m.setattr(gemm, name, record)
+        res = fn()
+    assert len(made) == 1 and made[0] is not None
+    return res
+
+
+def _shared(monkeypatch, fn):
+    """Whether CTAs share tiles in this call: the launcher asks for scratch."""
+    descs = []
+    with monkeypatch.context() as m:
+        m.setattr(gemm, "_launch", lambda d: descs.append(dict(d, cta_pair=gemm.CTA_PAIR)))
+        _alone(monkeypatch, fn)
+    return _native.lib().gemm_workspace(descs[0]) > 0
+
+
 @pytest.mark.parametrize("rows", [1, 31, 32, 33, 63, 64, 65])
 @pytest.mark.parametrize("groups,K,N,layout", [(1, 520, 8, "nk"), (1, 4096, 264, "nk"), (3, 128, 136, "kn"),
                                                (8, 1024, 512, "kn"), (1, 72, 128, "kn"), (8, 4096, 4096, "kn"),
@@ -42,9 +66,12 @@ def test_store(monkeypatch, rows, groups, K, N, layout):
 
     def run(dtype):
         return gemm.grouped_gemm(a, b, b_layout=layout, uniform_rows=rows, out_dtype=dtype, alpha=0.5)
-    for got in (run(torch.float32), _alone(monkeypatch, lambda: run(torch.float32))):
+    # 2 and 51 tiles with sums of 64 and 128 blocks; the others go round once as evenly or have short sums
+    shares = {(1, 4096): rows <= 32, (3, 8192): rows <= 64}.get((groups, K), False)
+    assert _shared(monkeypatch, lambda: run(None)) == shares
+    for got in (_taken(monkeypatch, lambda: run(torch.float32)), _alone(monkeypatch, lambda: run(torch.float32))):
         _close(got, 0.5 * want, 1e-5)
-    for got in (run(None), _alone(monkeypatch, lambda: run(None))):
+    for got in (_taken(monkeypatch, lambda: run(None)), _alone(monkeypatch, lambda: run(None))):
         _close(got, 0.5 * want, 4e-3)
     gemm.check_status()
 
@@ -80,9 +107,10 @@ def test_narrow_products_in_row_chunks(monkeypatch, rows, K, N, layout):
 
     def run(dtype):
         return gemm.grouped_gemm(a, b, b_layout=layout, uniform_rows=rows, out_dtype=dtype)
-    for got in (run(torch.float32), _alone(monkeypatch, lambda: run(torch.float32))):
+    assert _shared(monkeypatch, lambda: run(None)) == (K == 4096 and rows <= 100)      # 1000 rows go the other way
+    for got in (_taken(monkeypatch, lambda: run(torch.float32)), _alone(monkeypatch, lambda: run(torch.float32))):
         _close(got, want, 1e-5)
-    _close(run(None), want, 4e-3)
+    _close(_taken(monkeypatch, lambda: run(None)), want, 4e-3)
     gemm.check_status()
 
 
@@ -90,7 +118,8 @@ def test_narrow_products_in_row_chunks(monkeypatch, rows, K, N, layout):
 @pytest.mark.parametrize("rows,groups,K,F,probs,save", [(16, 8, 1024, 200, True, True), (32, 2, 128, 128, False, False),
                                                         (5, 3, 4096, 384, True, False), (17, 8, 2048, 3000, True, True),
                                                         (33, 3, 2048, 200, True, True), (64, 8, 1024, 1000, True, False),
-                                                        (49, 2, 128, 128, False, True), (65, 2, 192, 136, True, True)])
+                                                        (49, 2, 128, 128, False, True), (65, 2, 192, 136, True, True),
+                                                        (61, 3, 4096, 200, True, True)])
 def test_activation(monkeypatch, activation, rows, groups, K, F, probs, save):
     torch.manual_seed(1)
     a, w = _r(groups * rows, K), _r(groups, K, F * (2 if activation == "swiglu" else 1))
@@ -100,7 +129,10 @@ def test_activation(monkeypatch, activation, rows, groups, K, F, probs, save):
 
     def run():
         return gemm.grouped_gemm_act(a, w, p, activation=activation, uniform_rows=rows, save_pre=save)
-    for act, kept in (run(), _alone(monkeypatch, run)):
+    # 9, 6 and 192 tiles of 64 and 32 blocks; 6 of 32 blocks where a block is 36 KB
+    assert _shared(monkeypatch, run) == ((groups, K) in ((3, 4096), (8, 2048)) or
+                                         (groups, K, activation) == (3, 2048, "swiglu"))
+    for act, kept in (_taken(monkeypatch, run), _alone(monkeypatch, run)):
         _close(act, want, 4e-3)
         assert (kept is None) == (not save)
         if save:
@@ -109,22 +141,34 @@ def test_activation(monkeypatch, activation, rows, groups, K, F, probs, save):
 
 
 @pytest.mark.parametrize("rows", [16, 60])
-def test_repeats_streams_and_graphs(rows):
+def test_repeats_streams_and_graphs(monkeypatch, rows):
     """Shared tiles are summed in the order of their parts: every launch gives the same bytes, also more launches than
-    there are counter sets, on two streams in turn and from a captured graph."""
+    there are counter sets, from two streams at once, products of other sizes between them, and from a captured graph."""
     torch.manual_seed(3)
     a, w = _r(8 * rows, 2048), _r(8, 2048, 2 * 3072)
-    first = gemm.grouped_gemm_act(a, w, None, activation="swiglu", uniform_rows=rows, save_pre=False)[0].clone()
-    side = torch.cuda.Stream()
+    a2, w2 = _r(100, 4096), _r(64, 4096)
+
+    def run():
+        return gemm.grouped_gemm_act(a, w, None, activation="swiglu", uniform_rows=rows, save_pre=False)[0]
+
+    def other():
+        return gemm.grouped_gemm(a2, w2, b_layout="nk", uniform_rows=100, out_dtype=torch.float32)
+    assert _shared(monkeypatch, run) and _shared(monkeypatch, other)
+    first, second = run(), other()
+    # nothing is read on the host before all is queued: launches of both streams are under way together
+    side, got = torch.cuda.Stream(), []
     side.wait_stream(torch.cuda.current_stream())
     for i in range(150):
-        with torch.cuda.stream(side if i % 2 else torch.cuda.current_stream()):
-            got = gemm.grouped_gemm_act(a, w, None, activation="swiglu", uniform_rows=rows, save_pre=False)[0]
-            assert torch.equal(got, first)
-    torch.cuda.current_stream().wait_stream(side)
+        for stream in (side, torch.cuda.current_stream()):
+            with torch.cuda.stream(stream):
+                got.append((run(), first))
+                if i % 3 == 0:
+                    got.append((other(), second))
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, y) for x, y in got)
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
-        out = gemm.grouped_gemm_act(a, w, None, activation="swiglu", uniform_rows=rows, save_pre=False)[0]
+        out = run()
     for _ in range(3):
         out.zero_()
         graph.replay()

@@ -35,9 +35,31 @@ def _same(x, y, exact=True):
             assert (x - y).abs().max() <= 1e-5 * y.abs().max()
 
 
+@contextlib.contextmanager
+def _recorded(monkeypatch):
+    """Names of the C++ calls in the order made, with whether they took their arguments."""
+    made = []
+
+    def recorder(name, call):
+        def run(*args):
+            res = call(*args)
+            made.append((name, res is not None))
+            return res
+        return run
+    with monkeypatch.context() as m:
+        for mod in (gemm, elementwise, flash):
+            for name in [n for n in vars(mod) if n.startswith("_t_")]:
+                m.setattr(mod, name, recorder(name, getattr(mod, name)))
+        yield made
+
+
 def _both(monkeypatch, fn, exact=True, native=True):
+    """``fn`` by a C++ call and by the general path: the same results.  ``native``: the call takes this form; else it
+    hands it back, and the general path does it both times."""
     before = gemm.LAUNCHES + elementwise.LAUNCHES + flash.LAUNCHES
-    got = fn()
+    with _recorded(monkeypatch) as made:
+        got = fn()
+    assert made and all(taken == native for _, taken in made), made
     mid = gemm.LAUNCHES + elementwise.LAUNCHES + flash.LAUNCHES
     with _general(monkeypatch):
         want = fn()
@@ -94,9 +116,9 @@ def test_gemm_forms(monkeypatch, layout, form):
             return got[:64], got[64:69], got[128:188]
         return got
     if form == "grouped_hole":
-        before = gemm.LAUNCHES
-        got = run()
-        assert gemm.LAUNCHES == before + 1
+        with _recorded(monkeypatch) as made:
+            got = run()
+        assert made == [("_t_gemm", True)]
         with _general(monkeypatch):
             _same([g.clone() for g in got], [g.clone() for g in run()])
         return
@@ -151,22 +173,22 @@ def test_norm_forms(monkeypatch, T, kind, bias, residual):
     dy, res = _r(T, 264), _r(T, 264) if residual else None
     _both(monkeypatch, lambda: norm.norm_bwd(dy, x, w, mean, rstd, kind, bias, res))
     wide = _r(T, 528)[:, :264]                     # a strided gradient takes the general path
-    _both(monkeypatch, lambda: norm.norm_bwd(wide, x, w, mean, rstd, kind, bias, res))
+    _both(monkeypatch, lambda: norm.norm_bwd(wide, x, w, mean, rstd, kind, bias, res), native=T == 1)
 
 
 def test_row_and_routing_forms(monkeypatch):
     torch.manual_seed(4)
     x, idx = _r(50, 72), torch.randint(0, 50, (77,), device="cuda")
     _both(monkeypatch, lambda: elementwise.gather_rows(x, idx))
-    _both(monkeypatch, lambda: elementwise.gather_rows(x, idx.int()))
+    _both(monkeypatch, lambda: elementwise.gather_rows(x, idx.int()), native=False)
     _both(monkeypatch, lambda: elementwise.gather_rows(x, idx, torch.empty(77, 72, device="cuda", dtype=BF)))
     slot = torch.randint(-1, 50, (33, 3), device="cuda", dtype=torch.int32)
     res = _r(33, 72)
     _both(monkeypatch, lambda: elementwise.unpermute_reduce(x, slot, res))
-    _both(monkeypatch, lambda: elementwise.unpermute_reduce(x, slot.long()))
+    _both(monkeypatch, lambda: elementwise.unpermute_reduce(x, slot.long()), native=False)
     logits = _r(40, 16, dtype=F32)
     _both(monkeypatch, lambda: elementwise.topk_softmax(logits, 3))
-    _both(monkeypatch, lambda: elementwise.topk_softmax(_columns(logits), 3))
+    _both(monkeypatch, lambda: elementwise.topk_softmax(_columns(logits), 3), native=False)
     top, pr = elementwise.topk_softmax(logits, 3)
     _both(monkeypatch, lambda: elementwise.moe_plan(top, pr, 16, 8))
 
