@@ -77,8 +77,8 @@ int fm_cross_entropy(void* logits, const long long* labels, float* loss_out, int
                      float grad_scale, cudaStream_t s);
 
 // Router weight gradient dw [H, E] fp32 = x[T, H]^T (bf16) * dlogits[T, E] (fp32).  `partial` holds
-// fm_router_wgrad_splits(T, H, E) x H x E floats.
-int fm_router_wgrad_splits(int T, int H, int E);
+// fm_router_wgrad_splits(T, H, E, x on 16 bytes) x H x E floats.
+int fm_router_wgrad_splits(int T, int H, int E, int x_on_16);
 int fm_router_wgrad(const void* x, const float* dlogits, float* partial, float* dw, int T, int H, int E,
                     int* status, cudaStream_t s);
 // main[ids[t]] += dy[t] (fp32 rows of H values, bf16 gradients).  An id outside [0, rows) is left out and

@@ -249,7 +249,7 @@ def router_wgrad(x, dlogits):
     E = dlogits.shape[1]
     dlogits = dlogits.contiguous()
     lib = _native.lib()
-    partial = torch.empty(lib.router_wgrad_splits(T, H, E), H, E, dtype=torch.float32, device=x.device)
+    partial = torch.empty(lib.router_wgrad_splits(T, H, E, int(x.data_ptr() % 16 == 0)), H, E, dtype=torch.float32, device=x.device)
     dw = torch.empty(H, E, dtype=torch.float32, device=x.device)
     LAUNCHES += 1
     lib.router_wgrad(x.data_ptr(), dlogits.data_ptr(), partial.data_ptr(), dw.data_ptr(), T, H, E,

@@ -26,3 +26,13 @@ def test_head_split_divides_the_group(s, groups, per_group):
     tiles = -(-s // 128)
     if tiles * per_group * 148 * 2 <= 3 * groups * per_group * tiles * (tiles + 1) // 2:
         assert split == 1
+
+
+@pytest.mark.parametrize("T", [1, 500, 1535, 1536, 8192])
+@pytest.mark.parametrize("H,E", [(1024, 8), (4096, 8), (2048, 64), (8, 1)])
+def test_router_gradient_off_16_bytes_keeps_its_shares(T, H, E):
+    """Rows that the tensor core does not take: two CTAs an SM, of at least 32 tokens each, whatever their number."""
+    tiles = -(-H // 1024) * -(-E // (8 if E <= 8 else 16))
+    assert _C.router_wgrad_splits(T, H, E, 0) == max(1, min(2 * 148 // tiles, -(-T // 32)))
+    if T < 1536:
+        assert _C.router_wgrad_splits(T, H, E, 1) == _C.router_wgrad_splits(T, H, E, 0)
