@@ -99,17 +99,6 @@ constexpr int few_smem() {
   return few_stages<kKind, NT>() * few_stage_bytes<kKind, NT>() + 1024 + 512;
 }
 
-// 32 lanes x 16 consecutive fp32 columns.
-__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, float* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), "=f"(r[8]),
-        "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
-
 template <int kKind, bool kMn, int NT>
 __global__ void __launch_bounds__(kFewThreads, 1)
 gemm_few_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant__ CUtensorMap tma_x, const FewArgs a) {

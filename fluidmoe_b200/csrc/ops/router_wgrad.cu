@@ -4,17 +4,20 @@
 // On the fp32 pipe 8192 x 2048 x 64 takes 31 us at best, and took 80.  An fp32 gradient is exactly the sum of three bf16
 // numbers (8 + 8 + 8 bits), and a product of two bf16 numbers is exact in fp32, so three bf16 products give every bit
 // that one fp32 product gives.  What the tensor core does otherwise is to add: it cuts sums off where the fp32 pipe
-// rounds them.  Its sums are therefore kept short, 64 tokens each, and added up in registers; the leading part and the two
-// small ones have accumulators of their own.  Against 64-bit sums, relative, from
-// 2048 tokens on: terms of both signs 1.0e-7 to 1.7e-7 (fp32 pipe 1.8e-7 to 3.9e-7), of one sign 8.0e-8 to 9.8e-8
-// (9.2e-8 to 1.7e-7).
+// rounds them, which shows in sums of one sign.  Its sums are therefore kept short, two of 32 tokens for the leading part and one
+// of 64 for the two small ones, and added up in registers.  Against 64-bit sums, relative, 1536 to 8192 tokens, 512 to 4096
+// columns, 8 to 64 experts: terms of both signs 8.3e-8 to 1.3e-7 (fp32 pipe 1.6e-7 to 3.1e-7), of one sign 5.5e-8 to 1.0e-7
+// (8.5e-8 to 2.5e-7).  With one sum of 64 tokens for the leading part too, terms of one sign were off by up to 1.4 times as
+// much as on the fp32 pipe; the time is the same.
 // A CTA owns 128 columns of x (the M of the product; x is read by TMA as it lies, token-major), up to 64 experts and a
 // share of the tokens.  Eight warps cut the gradients of 64 tokens into their parts and write them in the layout of the
 // product's other operand, four add up finished sums, so that the tensor core has the next block meanwhile.  The
 // shares of the tokens are summed in a fixed order by a second kernel.
-// Both kernels, fp32 pipe and this, us: 8192 x 2048 x 64 85 and 27.6; x 128 155 and 42; 8192 x 1024 x 160 103 and 34;
-// 4096 x 2048 x 16 29.7 and 17.4; 4096 x 4096 x 8 25.6 and 23.5; 16384 x 4096 x 8 64.5 and 60.4; 2048 x 1024 x 8 17.4 and 13.2.
+// Both kernels, fp32 pipe and this, us: 8192 x 2048 x 64 95 and 29.7; x 128 173 and 44; 8192 x 1024 x 160 115 and 38;
+// 4096 x 2048 x 16 34 and 19.5; 4096 x 4096 x 8 29.7 and 23.6; 16384 x 4096 x 8 69 and 58; 2048 x 1024 x 8 19.3 and 15.1.
 #include <cuda_bf16.h>
+
+#include <algorithm>
 
 #include "../include/fm_tmap.h"
 #include "../include/sm100_ptx.cuh"
@@ -29,6 +32,8 @@ constexpr int kRwRows = 128, kRwCols = 64, kRwTokens = 64, kRwStages = 4, kRwPar
 constexpr int kRwBoxBytes = 64 * 64 * 2;                                   // 64 tokens of 64 columns or experts
 constexpr int kRwStageBytes = (kRwRows / 64 + kRwParts) * kRwBoxBytes;
 constexpr int kRwSmem = kRwStages * kRwStageBytes + 1024 + 256;
+constexpr int kRwChains = 2;          // accumulators of the leading part: sums of 32 tokens each
+constexpr int kRwAccCols = (kRwChains + 1) * kRwCols, kRwTmemCols = 512;   // twice 192, allocated by powers of two
 constexpr int kKernelIdRouterWgrad = 4;
 
 // Eight gradients as three bf16 vectors.  Truncation keeps every part finite; what is not finite is all in the first.
@@ -81,7 +86,7 @@ router_wgrad_mma_kernel(const __grid_constant__ CUtensorMap tma_x, const float* 
     tma_prefetch_desc(&tma_x);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 256);
+    tmem_alloc(tmem_slot, kRwTmemCols);
     tmem_relinquish();
   }
   tc_fence_before_sync();
@@ -120,15 +125,16 @@ router_wgrad_mma_kernel(const __grid_constant__ CUtensorMap tma_x, const float* 
       tc_fence_after_sync();
       if (elect_one()) {
         const uint32_t x0 = smem_u32(smem + st * kRwStageBytes), g0 = x0 + 2 * kRwBoxBytes;
-        const uint32_t lead = tmem_base + acc * 128, rest = lead + kRwCols;
+        const uint32_t lead = tmem_base + acc * kRwAccCols, rest = lead + kRwChains * kRwCols;
+        constexpr int kChain = kRwTokens / 16 / kRwChains;       // products of a chain
 #pragma unroll
         for (int k = 0; k < kRwTokens / 16; ++k) {
           const uint64_t x = umma_desc_join(umma_desc_lo(x0 + k * 2048, kRwBoxBytes), kDescHi);
 #pragma unroll
           for (int p = 0; p < kRwParts; ++p)
-            umma_bf16(p == 0 ? lead : rest, x,
+            umma_bf16(p == 0 ? lead + k / kChain * kRwCols : rest, x,
                       umma_desc_join(umma_desc_lo(g0 + p * kRwBoxBytes + k * 2048, kRwBoxBytes), kDescHi), idesc,
-                      k > 0 || p == 2 ? 1u : 0u);
+                      (p == 0 ? k % kChain > 0 : k > 0 || p == 2) ? 1u : 0u);
         }
         umma_commit(&empty[st]);
         umma_commit(&tfull[acc]);
@@ -190,17 +196,19 @@ router_wgrad_mma_kernel(const __grid_constant__ CUtensorMap tma_x, const float* 
       if (!wait_all(&tfull[acc], (j >> 1) & 1, 500 + acc)) break;
       tc_fence_after_sync();
 #pragma unroll
-      for (int c = 0; c < kRwCols / 32; ++c) {
-        if (c * 32 >= cols) continue;
-        uint32_t a[32], b[32];
-        tmem_ld_32x32(tmem_base + lane_addr + acc * 128 + c * 32, a);
-        tmem_ld_32x32(tmem_base + lane_addr + acc * 128 + kRwCols + c * 32, b);
+      for (int c = 0; c < kRwCols / 16; ++c) {
+        if (c * 16 >= cols) continue;
+        const uint32_t t = tmem_base + lane_addr + acc * kRwAccCols + c * 16;
+        float a[kRwChains][16], b[16];
+#pragma unroll
+        for (int i = 0; i < kRwChains; ++i) tmem_ld_32x16(t + i * kRwCols, a[i]);
+        tmem_ld_32x16(t + kRwChains * kRwCols, b);
         tmem_ld_wait();
 #pragma unroll
-        for (int e = 0; e < 32; ++e) {
+        for (int e = 0; e < 16; ++e) {
           // an infinity in x meets the zeros of the small parts: the leading sum alone tells
-          const float lead = __uint_as_float(a[e]);
-          sum[c * 32 + e] += fabsf(lead) < INFINITY ? lead + __uint_as_float(b[e]) : lead;
+          const float lead = a[0][e] + a[1][e];
+          sum[c * 16 + e] += fabsf(lead) < INFINITY ? lead + b[e] : lead;
         }
       }
       tc_fence_before_sync();
@@ -232,21 +240,24 @@ router_wgrad_mma_kernel(const __grid_constant__ CUtensorMap tma_x, const float* 
   __syncthreads();
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, 256);
+    tmem_dealloc(tmem_base, kRwTmemCols);
   }
 }
 
 static int rw_tiles(int H, int E) { return ((H + kRwRows - 1) / kRwRows) * ((E + kRwCols - 1) / kRwCols); }
 static int rw_per_split(int T, int H, int E) {
-  const int want = 148 / rw_tiles(H, E), splits = want < 1 ? 1 : want;
+  // One round of CTAs; but a lane adds up the blocks of a share one after another, so two shares at the least and no share
+  // of more than 4096 tokens.
+  const int splits = std::max({148 / rw_tiles(H, E), 2, (T + 4095) / 4096});
   const int per = (T + splits - 1) / splits;
   return (per + kRwTokens - 1) / kRwTokens * kRwTokens;
 }
 
-// From 1536 tokens on: below that the fp32 pipe rounds few sums (one sign, 512 x 2048 x 64: 6.5e-8 against 8.3e-8) and
-// there is little to gain (17.4 and 15.1 us).  One round of CTAs, and rows that TMA takes.
+// From 1536 tokens on: below that the fp32 pipe rounds few sums (one sign, 512 x 2048 x 64: 6.5e-8) and there is little to
+// gain (17.4 and 15.1 us).  Up to 256 columns the fp32 pipe has more and shorter shares (one sign, 4096 x 128 x 128: 9.9e-8 and
+// 1.3e-7).  No more tiles than SMs, and rows that TMA takes.
 bool router_wgrad_mma_applies(int T, int H, int E) {
-  return H % 8 == 0 && rw_tiles(H, E) <= 148 && T >= 1536;
+  return H % 8 == 0 && H > 2 * kRwRows && rw_tiles(H, E) <= 148 && T >= 1536;
 }
 int router_wgrad_mma_splits(int T, int H, int E) {
   const int per = rw_per_split(T, H, E);

@@ -585,7 +585,7 @@ dropless_place_kernel(const long long* __restrict__ top_idx, const float* __rest
 
 // --------------------------------------------------------------------------------------------
 // Router weight gradient dW[h, e] = sum_t x[t, h] * dlogits[t, e], x in bf16, everything else fp32, where the
-// tensor core does not do it (router_wgrad.cu: few tokens, rows that TMA does not take).  A CTA owns 1024
+// tensor core does not do it (router_wgrad.cu: few tokens or columns, rows that TMA does not take).  A CTA owns 1024
 // columns of x (a thread four neighbours), EB experts and a share of the tokens; the gradients of the
 // logits are the same for all threads and come from shared memory four at a time.  The shares are summed in
 // a fixed order by a second kernel.  Against a conversion of x to fp32 and a library product, with a third of the
