@@ -11,7 +11,7 @@
 // fp32 by the last of them to arrive, in the order of its parts (no CTA waits for another).
 // Reading weights at 6.1 TB/s, 0.93 of the measured copy rate, for 8 groups of 16 rows, 4096 -> 2 x 14336 (360 -> 307 us);
 // 5.4 TB/s for 14336 -> 4096 (181 -> 174), whose rows of 8 KB are cut into pieces of 512 bytes.  The pass over 64 tokens
-// of a Mixtral-sized MoE, which the power of the wide products had slowed besides: 697 -> 508 us.
+// of a Mixtral-sized MoE, which the power of the wide products had slowed besides: 703 -> 503 us.
 // The same product as the tiled GEMM's with store or activation epilogue; the counterpart in the reference are its per-expert
 // products (fluid/moe/forward.py:217-352).
 #include <cuda_bf16.h>

@@ -455,7 +455,7 @@ __device__ __forceinline__ void get_block_bf16(float* stg, int lane, float* v, i
 // one pipeline stage less, 8 experts of 1024 rows take 3.70 -> 2.69 ms for 4096 x 28672 and 1.78 -> 1.32 ms for
 // 14336 x 4096.
 // Parameter and moments are not fetched into L2 ahead of the boxes: a tile ahead on every SM is 58 MB of lines on their
-// way, which pushed each other and the operands out (1.38 GB read for 0.94); 2.81 -> 2.66 ms and 1.38 -> 1.29 without,
+// way, which pushed each other and the operands out (8 x 4096 x 7168: 2.38 GB read for 1.59, without 1.73); 2.81 -> 2.66 ms and 1.38 -> 1.29 without,
 // the activation's gradient, which did the same, 765 -> 720, 292 -> 267 and 288 -> 251 us for the sizes below.
 // ----------------------------------------------------------------------------------------
 struct EpiAdam {

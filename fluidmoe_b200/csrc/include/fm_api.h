@@ -98,7 +98,8 @@ typedef struct FmGemmDesc {
   long long workspace_bytes;
 } FmGemmDesc;
 
-// Returns 0 on success, a cudaError_t / negative code otherwise.  Never allocates.
+// Returns 0 on success, a cudaError_t / negative code otherwise.  Allocates nothing but, once for each of the first 64 streams
+// and when its tiles become more, the counters and the tile log that the launches of a stream share.
 int fm_gemm_launch(const FmGemmDesc* d, cudaStream_t stream);
 // Bytes of scratch that make this launch faster (0 for most).
 long long fm_gemm_workspace(const FmGemmDesc* d);

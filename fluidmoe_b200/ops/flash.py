@@ -64,7 +64,7 @@ def _head_split(s: int, b: int, groups: int, q_per_group: int, sms: int = 148) -
 
     A CTA walks the query tiles behind its block for each of its heads, so the CTA of the first block is the longest.
     Heads are split until it takes no more than one and a half times an SM's share of all steps; a further split only
-    adds the fp32 sums of dK and dV, a fill and a conversion.  One against two and four CTAs, 8 KV heads of 4: 4096
+    adds the fp32 sums of dK and dV and a conversion.  One against two and four CTAs, 8 KV heads of 4: 4096
     positions (longest 128 steps, share 114) 345, 378, 415 us; 3072 (96, 65) 253, 247, 265; 2048 (64, 29) 171, 134, 155;
     1024 (32, 8) 93, 73, 69.  1 of 8, 4096 (256, 29): 548, 289, 165, eight CTAs 110."""
     tiles = (s + 127) // 128

@@ -99,6 +99,23 @@ def case_fc1(a):
     return x, w, probs, act, pre
 
 
+def case_few(a):
+    """FC1 and FC2 of few rows an expert, which read every weight once."""
+    R, H, F, G = a.rows, a.hidden, a.ffn, a.experts
+    x, y, w1, w2 = _r(R, H), _r(R, F), _r(G, H, 2 * F, scale=0.02), _r(G, F, H, scale=0.02)
+    report(f"fc1 swiglu G={G}, {R // G} rows {H}x{2 * F}",
+           timed(lambda: gemm.grouped_gemm_act(x, w1, None, activation="swiglu", uniform_rows=R // G, save_pre=False)),
+           bytes_=w1.numel() * 2.0)
+    report(f"fc2 G={G}, {R // G} rows {F}x{H}", timed(lambda: gemm.grouped_gemm(y, w2, uniform_rows=R // G)),
+           bytes_=w2.numel() * 2.0)
+
+
+def case_router(a):
+    x, dl = _r(a.rows, a.hidden), torch.randn(a.rows, a.experts, device="cuda")
+    report(f"router weight gradient {a.rows}x{a.hidden}, {a.experts} experts", timed(lambda: ew.router_wgrad(x, dl)),
+           2.0 * a.rows * a.hidden * a.experts, a.rows * (a.hidden * 2.0 + a.experts * 4.0))
+
+
 def case_dact(a):
     R, H, F, G = a.rows, a.hidden, a.ffn, a.experts
     dy, w2, pre = _r(R, H), _r(G, F, H, scale=0.02), _r(R, 2 * F)
@@ -252,8 +269,8 @@ def case_fused(a):
     report(f"FC2 + combine (scatter epilogue) + unpermute {rows}x{F}x{H}", timed(fc2), 2.0 * rows * F * H)
 
 
-CASES = dict(gemm=case_gemm, fc1=case_fc1, dact=case_dact, wgrad=case_wgrad, wgrad_adam=case_wgrad_adam, flash=case_flash,
-             norm=case_norm, permute=case_permute, adam=case_adam, ce=case_ce, rope=case_rope, fused=case_fused)
+CASES = dict(gemm=case_gemm, fc1=case_fc1, few=case_few, router=case_router, dact=case_dact, wgrad=case_wgrad,
+             wgrad_adam=case_wgrad_adam, flash=case_flash, norm=case_norm, permute=case_permute, adam=case_adam, ce=case_ce, rope=case_rope, fused=case_fused)
 
 
 def main(argv=None):
@@ -271,7 +288,8 @@ def main(argv=None):
     ap.add_argument("--q-per-kv", type=int, default=4)
     ap.add_argument("--elems", type=int, default=1 << 28)
     ap.add_argument("--fwd-versions", type=int, nargs="+", default=[2, 1],
-                    help="attention forward kernels to time (2: default; 20..24: share of polynomial exponentials; 1: first generation)")
+                    help="attention forward kernels to time (0: by size; 2, 3: two query tiles a CTA and one; 20..24: share of "
+                         "polynomial exponentials; 1: first generation)")
     ap.add_argument("--bwd-versions", type=int, nargs="+", default=[2, 1])
     a = ap.parse_args(argv)
     torch.manual_seed(0)
