@@ -22,8 +22,9 @@ def status_buffer(device) -> torch.Tensor:
     key = str(device)
     if key not in _STATUS:
         _STATUS[key] = torch.zeros(8, dtype=torch.int32, device=device)
-        if _STATUS[key].is_cuda:
-            _STATUS_PTR.setdefault(_STATUS[key].get_device(), _STATUS[key].data_ptr())
+        # the words that ``check_status(tensor.device)`` reads: a device named without its index has words of its own
+        if _STATUS[key].is_cuda and key == str(_STATUS[key].device):
+            _STATUS_PTR[_STATUS[key].get_device()] = _STATUS[key].data_ptr()
     return _STATUS[key]
 
 

@@ -241,3 +241,17 @@ def test_deterministic_mode_still_fills(monkeypatch):
         assert out[8:].isnan().all()
     finally:
         torch.use_deterministic_algorithms(False)
+
+
+def test_status_words_are_those_of_the_tensor_s_device(monkeypatch):
+    """A call reports where ``check_status(tensor.device)`` looks, also when words for a device without an index came
+    first."""
+    monkeypatch.setattr(gemm, "_STATUS", {})
+    monkeypatch.setattr(gemm, "_STATUS_PTR", {})
+    x = _r(8, 8)
+    unnamed = gemm.status_buffer("cuda")
+    assert gemm.status_ptr(x) == gemm.status_buffer(x.device).data_ptr() != unnamed.data_ptr()
+    gemm.status_buffer(x.device)[0] = 1
+    gemm.check_status("cuda")
+    with pytest.raises(gemm.FluidKernelTimeout):
+        gemm.check_status(x.device)
